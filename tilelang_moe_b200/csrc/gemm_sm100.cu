@@ -412,7 +412,12 @@ __device__ __forceinline__ uint32_t pack_out(float a, float b, int f16) {
   }
   return pack_bf16(a, b);
 }
-__device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.0f + __expf(-g)) * u; }
+// The division is the fast intrinsic: at most 2 ulp of fp32, like __expf's, and both far below the 16-bit rounding of
+// the product.  What counts is that it has no slow path: lanes without a live row hold whatever tensor memory held, and the
+// checked division takes its out-of-line branch for such values, element by element, while the whole warp waits.
+// Measured (2 rows on 9 experts, H=2048, I=512): 37.9 us per launch with the checked division, 16.3 with this one; with
+// 341 rows per expert 41 -> 20 us.
+__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 
 // ------------------------------------------------------------------------------ kernel
 template <int MT, int BN, int EPI, bool GATHER>
