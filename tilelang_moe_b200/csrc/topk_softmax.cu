@@ -1,8 +1,9 @@
 // Fused top-k + softmax router kernels for sm_100a.
 //
-// Three kernels behind one entry point:
-//   * topk_tile_kernel   rows staged in shared memory by cp.async, 1-8 threads per row keep a sorted
-//                        k-entry list in registers; N <= 1024, k <= 8, aligned rows, M >= 64.
+// Four kernels behind one entry point:
+//   * topk_group_kernel  4-32 lanes per row, the row in their registers, a threshold from part maxima, then a ranking of
+//                        the few logits not below it; N <= 1024, k <= 8, aligned rows, M >= 2048 or N > 256.
+//   * topk_lane_kernel   the same with one lane per row, staged through shared memory; N <= 32.
 //   * topk_warp_kernel   one warp per row, the row lives in registers; k rounds of
 //                        warp-wide arg-max by redux; N <= 1024, k <= 64.
 //   * topk_radix_kernel  a thread-block cluster per row; each CTA stages its slice
@@ -11,7 +12,7 @@
 //                        keys with histograms combined over distributed shared
 //                        memory, the selected entries are gathered into the leading
 //                        CTA, sorted (bitonic, 64-bit key|index) and normalised.
-// Both read every logit exactly once from global memory.
+// All read every logit once from HBM.
 //
 // Ordering contract: descending by value, equal values lowest index first,
 // -0.0 == +0.0, NaN above every number.
@@ -139,204 +140,421 @@ static int launch_warp(const float* logits, int64_t M, int N, int64_t ld, int k,
 
 
 // ------------------------------------------------------------------------------------
-// thread-per-row kernel for small k (k <= 8, N <= 1024, 16-byte aligned rows)
+// lane-group kernel for small k (k <= 8, N <= 1024, N % 4 == 0, 16-byte aligned rows)
 //
-// A CTA of 128 threads stages a tile of rows in shared memory with 16-byte cp.async (coalesced, the only
-// read of the logits), then TPR = 1, 2, 4 or 8 adjacent threads share one row: each scans its part with a
-// sorted k-entry list in registers (compare against the k-th best, insert by a compare-exchange chain),
-// partial lists are merged over shuffles, and the first thread of the row normalises and writes.
-// The instruction cost per row is a quarter of the warp-per-row kernel's; three CTAs per SM keep ~190 KB of
-// loads in flight.  Keys are signed integers ordered like the floats: x + 0.0f folds -0.0 into +0.0 and every
-// NaN into the canonical positive NaN, which ranks above +inf.
+// L = 4 .. 32 neighbouring lanes share a row, EPT = 8 .. 32 logits per lane, straight from global memory into registers
+// with 16-byte loads (the only pass over the logits).  A row is never ordered as a whole:
+//   1. every lane takes the maxima of four parts of its logits; the group merges them over shuffles (sorted lists, the
+//      upper half kept) into V, the K-th largest of the 4 * L part maxima - a lower bound of the K-th largest logit;
+//   2. the logits not below V, seven or eight of them as a rule, are collected in shared memory as 64-bit key | column
+//      entries (equal keys: lowest column first);
+//   3. each lane ranks its share of them against all of them; the entries of rank < k are the result, in order.
+// NaNs do not enter V (max and min ignore them) and are never below it, so they are collected and rank first by key.
+// A warp with more than CAP entries in one of its rows takes the logits equal to V in column order, K at most; where
+// the logits above V alone are too many (rows sorted by expert, rows masked to -inf), every lane keeps a sorted list.
+//
+// What bounds it: instruction issue at N = 128, HBM from N = 512 on.  Few rows: the chain of one warp.  Measured (us,
+// thread-per-row tiles with a list of K per thread before -> now): 1048576 x 128, k = 6: 169 -> 138 (HBM 92);
+// 131072 x 256, k = 8: 65 -> 34; 131072 x 1024, k = 8: 291 -> 122 (HBM 83); 16384 x 256: 13.0 -> 7.9; 2048 x 256:
+// 9.0 -> 3.4; 131072 x 128 with all logits equal 24.6 -> 20.6, rounded to integers 28.7 -> 25.7.  With a few lanes per
+// row 32 warps per SM fit beside each other; the tiles had 12.
 // ------------------------------------------------------------------------------------
-constexpr int TILE_THREADS = 128;
-constexpr int MAX_PART_VECS = 32;   // 16-byte vectors one thread scans: at most 128 floats of a row per thread
+constexpr int GROUP_WARPS = 8;
 
+__device__ __forceinline__ void ce_desc(float& a, float& b) {
+  const float hi = fmaxf(a, b), lo = fminf(a, b);
+  a = hi; b = lo;
+}
+// s is bitonic: sorts it descending
+template <int P>
+__device__ __forceinline__ void bitonic_merge_desc(float (&s)[P]) {
+#pragma unroll
+  for (int st = P / 2; st > 0; st >>= 1)
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+      if ((i & st) == 0) ce_desc(s[i], s[i | st]);
+}
 
-template <int K, int TPR>
-__global__ void __launch_bounds__(TILE_THREADS)
-topk_tile_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld, int k, int mode, int rows_per_tile,
-                 float* __restrict__ scores, int64_t* __restrict__ idx64, int32_t* __restrict__ idx32) {
-  extern __shared__ __align__(16) float tile[];
-  __shared__ unsigned char queue[(2 * K - 1) * TILE_THREADS];   // per thread: vectors that can hold one of its K largest
-  const int tid = threadIdx.x;
-  const int pitch = N + 4;                         // floats; 16-byte aligned rows, conflict-free 16-byte reads
-  const int vec_per_row = N >> 2;
-  const int row_in_tile = tid / TPR, part = tid % TPR;
-  const int part_vecs = (vec_per_row + TPR - 1) / TPR;
-  const int64_t n_tiles = (M + rows_per_tile - 1) / rows_per_tile;
-  // staging walk of this thread: first vector, and the step of 128 vectors in rows / columns / bytes
-  const int ld_r0 = tid / vec_per_row, ld_c0 = tid % vec_per_row;
-  const int ld_dr = TILE_THREADS / vec_per_row, ld_dc = TILE_THREADS % vec_per_row;
-  const int64_t ld_dsrc = (int64_t)ld_dr * ld + ld_dc * 4;
-  const uint32_t ld_ddst = (uint32_t)(ld_dr * pitch + ld_dc * 4) * 4u;
-  const uint32_t tile_s = (uint32_t)__cvta_generic_to_shared(tile);
+template <int K, int L, int EPT>
+__global__ void __launch_bounds__(GROUP_WARPS * 32, EPT == 32 ? 4 : 5)
+topk_group_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld, int k, int mode,
+                  float* __restrict__ scores, int64_t* __restrict__ idx64, int32_t* __restrict__ idx32) {
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  constexpr int RPW = 32 / L;                       // rows per warp
+  constexpr int CAP = L == 32 ? 32 : 16;            // entries a row may collect
+  constexpr int HELD = CAP / L;                     // entries a lane ranks
+  constexpr int P = K > 4 ? 8 : (K > 2 ? 4 : 2);    // length of the merged lists of maxima
+  constexpr int PART = EPT / 4;
+  __shared__ uint64_t cand_s[GROUP_WARPS][RPW][CAP + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sub = lane & (L - 1), rw = lane / L;
+  const int64_t row0 = ((int64_t)blockIdx.x * GROUP_WARPS + warp) * RPW;
+  if (row0 >= M) return;                            // whole warps only: no block barrier below
+  const int64_t row = row0 + rw;
+  const bool live = row < M;
+  const float* p = logits + (live ? row : M - 1) * ld;
+  uint64_t* cand = cand_s[warp][rw];
+  const float NEG_INF = __int_as_float((int)0xFF800000);
 
-  for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-    const int64_t row0 = t * rows_per_tile;
-    const int rows = (int)((M - row0) < rows_per_tile ? (M - row0) : rows_per_tile);
-    __syncthreads();                               // previous tile fully consumed
-    {   // thread t copies vectors t, t + 128, ... of the tile; (row, column) advance by a fixed step, no division
-      int r = ld_r0, c = ld_c0;
-      const float* src = logits + (row0 + r) * ld + c * 4;
-      uint32_t dst = tile_s + (uint32_t)(r * pitch + c * 4) * 4u;
-      while (r < rows) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-        r += ld_dr; c += ld_dc;
-        src += ld_dsrc; dst += ld_ddst;
-        if (c >= vec_per_row) { c -= vec_per_row; r += 1; src += ld - N; dst += (uint32_t)(pitch - N) * 4u; }
-      }
+  // logits 4i .. 4i+3 of this lane are columns 4 * (i * L + sub) ...: a group reads 16 * L consecutive bytes at a time
+  float x[EPT];
+  uint32_t valid = 0u;
+#pragma unroll
+  for (int i = 0; i < EPT / 4; ++i) {
+    const int col = 4 * (i * L + sub);
+    if (col < N) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p + col));
+      x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+      valid |= 0xFu << (4 * i);
+    } else {
+      x[4 * i] = x[4 * i + 1] = x[4 * i + 2] = x[4 * i + 3] = NEG_INF;
     }
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
+  }
 
-    const bool active = row_in_tile < rows;
+  // ---- 1. V
+  float g[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float m = NEG_INF;
+#pragma unroll
+    for (int j = 0; j < PART; ++j) m = fmaxf(m, x[q * PART + j]);
+    g[q] = m;
+  }
+  ce_desc(g[0], g[1]); ce_desc(g[2], g[3]); ce_desc(g[0], g[2]); ce_desc(g[1], g[3]); ce_desc(g[1], g[2]);
+  float s[P];
+  if (P == 8) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { s[i] = g[i]; s[P - 1 - i] = __shfl_xor_sync(FULL, g[i], 1); }
+    bitonic_merge_desc<P>(s);
+  } else {
+#pragma unroll
+    for (int i = 0; i < P; ++i) s[i] = g[i];
+  }
+#pragma unroll
+  for (int d = P == 8 ? 2 : 1; d < L / 2; d <<= 1) {
+    float o[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) o[i] = __shfl_xor_sync(FULL, s[i], d);
+#pragma unroll
+    for (int i = 0; i < P; ++i) s[i] = fmaxf(s[i], o[P - 1 - i]);
+    bitonic_merge_desc<P>(s);
+  }
+  float V;
+  {   // K-th largest of two descending lists: the best split into i entries of one and K - i of the other
+    float o[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) o[i] = __shfl_xor_sync(FULL, s[i], L / 2);
+    V = fmaxf(s[K - 1], o[K - 1]);
+#pragma unroll
+    for (int i = 1; i < K; ++i) V = fmaxf(V, fminf(s[i - 1], o[K - i - 1]));
+  }
+
+  // ---- 2. collect
+  uint32_t mask = 0u;
+#pragma unroll
+  for (int b = 0; b < EPT; ++b) mask |= !(x[b] < V) ? (1u << b) : 0u;
+  mask &= valid;
+  int mine_n = __popc(mask);
+  int inc = mine_n;
+#pragma unroll
+  for (int d = 1; d < L; d <<= 1) {
+    const int v = __shfl_up_sync(FULL, inc, d, L);
+    if (sub >= d) inc += v;
+  }
+  int c = __shfl_sync(FULL, inc, L - 1, L);
+  int cmax = __reduce_max_sync(FULL, c);
+  if (cmax > CAP) {
+    // many logits equal to V: collect those above it and, one column at a time, the first K of the equal ones
+    uint32_t eq = 0u;
+#pragma unroll
+    for (int b = 0; b < EPT; ++b) eq |= x[b] == V ? (1u << b) : 0u;
+    eq &= mask;
+    mask &= ~eq;
+    mine_n = __popc(mask);
+    inc = mine_n;
+#pragma unroll
+    for (int d = 1; d < L; d <<= 1) {
+      const int v = __shfl_up_sync(FULL, inc, d, L);
+      if (sub >= d) inc += v;
+    }
+    c = __shfl_sync(FULL, inc, L - 1, L);
+    cmax = __reduce_max_sync(FULL, c);
+    if (cmax <= CAP - K) {
+      const uint64_t vkey = (uint64_t)float_to_key(V) << 32;
+      for (int r = 0; r < K; ++r) {
+        const int b = __ffs(eq) - 1;
+        const uint32_t col = eq ? (uint32_t)(4 * ((b >> 2) * L + sub) + (b & 3)) : 0xFFFFFFFFu;
+        uint32_t first = col;
+#pragma unroll
+        for (int d = 1; d < L; d <<= 1) first = min(first, __shfl_xor_sync(FULL, first, d));
+        if (first != 0xFFFFFFFFu) {
+          if (col == first) {
+            cand[c] = vkey | (uint64_t)(0xFFFFFFFFu - col);
+            eq &= eq - 1;
+          }
+          ++c;
+        }
+      }
+      cmax = __reduce_max_sync(FULL, c);
+    } else {
+      cmax = CAP + 1;
+    }
+  }
+  if (cmax <= CAP) {
+    int slot = inc - mine_n;
+    while (mask) {                                  // the value comes from L1 again: registers have no dynamic index
+      const int b = __ffs(mask) - 1;
+      mask &= mask - 1;
+      const int col = 4 * ((b >> 2) * L + sub) + (b & 3);
+      cand[slot++] = ((uint64_t)float_to_key(__ldg(p + col)) << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)col);
+    }
+    __syncwarp();
+    // ---- 3. rank
+    uint64_t mine[HELD];
+    int rank[HELD];
+#pragma unroll
+    for (int h = 0; h < HELD; ++h) {
+      const int q = h * L + sub;
+      mine[h] = q < c ? cand[q] : 0ull;
+      rank[h] = 0;
+    }
+    for (int j = 0; j < cmax; ++j) {
+      const uint64_t v = j < c ? cand[j] : 0ull;
+#pragma unroll
+      for (int h = 0; h < HELD; ++h)
+        if (h == 0 || h * L < cmax) rank[h] += v > mine[h] ? 1 : 0;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < HELD; ++h)
+      if (h * L + sub < c && rank[h] < k) cand[rank[h]] = mine[h];
+  } else {
+    // every lane keeps a sorted list of its K largest (columns ascend within a lane, so equal keys keep the lowest
+    // column first), then k rounds of arg-max over the heads of the group's lists
     int kv[K], ki[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) { kv[j] = (int)0x80000000; ki[j] = 0; }
-    const float* rowp = tile + row_in_tile * pitch;
-    const int v_lo = part * part_vecs, v_hi = min(vec_per_row, v_lo + part_vecs);
-    if (active) {
-      // Pass 1, branch-free: the largest key of every 4-element vector, and the K largest of those (keys only: a
-      // max / min pair per list entry).  The K largest elements of the part sit in vectors whose largest key is at
-      // least the K-th largest vector maximum V: at most K-1 vectors lie above V, and of those equal to V only the
-      // first K in column order can matter.
-      int vm[MAX_PART_VECS];
-      constexpr int CH = 2;                   // independent lists (two dependency chains in flight), one per half of the part
-      constexpr int QV = MAX_PART_VECS / CH;
-      int va[CH][K];
-#pragma unroll
-      for (int c = 0; c < CH; ++c)
-#pragma unroll
-        for (int j = 0; j < K; ++j) va[c][j] = (int)0x80000000;
-#pragma unroll
-      for (int u = 0; u < QV; ++u) {
-        int m[CH];
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          m[c] = (int)0x80000000;
-          if (v_lo + u + c * QV < v_hi) {
-            const float4 x = *reinterpret_cast<const float4*>(rowp + (v_lo + u + c * QV) * 4);
-            m[c] = max(max(float_to_ikey(x.x), float_to_ikey(x.y)), max(float_to_ikey(x.z), float_to_ikey(x.w)));
-          }
-          vm[u + c * QV] = m[c];
-        }
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-#pragma unroll
-          for (int c = 0; c < CH; ++c) {
-            const int hi = max(va[c][j], m[c]);
-            m[c] = min(va[c][j], m[c]);
-            va[c][j] = hi;
-          }
-        }
-      }
-#pragma unroll
-      for (int c = 1; c < CH; ++c) {          // the K largest of all lists end up in va[0]
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-          int m = va[c][i];
-#pragma unroll
-          for (int j = 0; j < K; ++j) {
-            const int hi = max(va[0][j], m);
-            m = min(va[0][j], m);
-            va[0][j] = hi;
-          }
-        }
-      }
-      // Pass 2, predicated: queue the vectors that can hold a winner (this thread's slots in shared memory)
-      const int V = va[0][K - 1];
-      int cnt = 0, n_eq = 0;
-#pragma unroll
-      for (int u = 0; u < MAX_PART_VECS; ++u) {
-        const bool eq = vm[u] == V && n_eq < K && v_lo + u < v_hi;
-        const bool take = (vm[u] > V) || eq;
-        if (take) queue[cnt * TILE_THREADS + tid] = (unsigned char)u;
-        cnt += take ? 1 : 0;
-        n_eq += eq ? 1 : 0;
-      }
-      // Pass 3: the queued vectors (about K of them) go through the sorted list with their columns, largest element
-      // first, lowest column first among equal ones
-      for (int q = 0; q < cnt; ++q) {
-        const int v = v_lo + (int)queue[q * TILE_THREADS + tid];
-        const float4 x = *reinterpret_cast<const float4*>(rowp + v * 4);
-        int c0 = float_to_ikey(x.x), c1 = float_to_ikey(x.y), c2 = float_to_ikey(x.z), c3 = float_to_ikey(x.w);
-        int m = max(max(c0, c1), max(c2, c3));
-        while (m >= V && m > kv[K - 1]) {     // nothing below V can be among the K largest: K vector maxima are >= V
-          const int sel = c0 == m ? 0 : (c1 == m ? 1 : (c2 == m ? 2 : 3));
-          list_insert<K>(kv, ki, m, v * 4 + sel);
-          c0 = sel == 0 ? (int)0x80000000 : c0;
-          c1 = sel == 1 ? (int)0x80000000 : c1;
-          c2 = sel == 2 ? (int)0x80000000 : c2;
-          c3 = sel == 3 ? (int)0x80000000 : c3;
-          m = max(max(c0, c1), max(c2, c3));
-        }
+#pragma unroll 1                                    // rolled, values from L1: unrolled it would cost the whole kernel registers
+    for (int i = 0; i < EPT / 4; ++i) {
+      const int col = 4 * (i * L + sub);
+      if (col < N) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p + col));
+        const int c0 = float_to_ikey(v.x), c1 = float_to_ikey(v.y), c2 = float_to_ikey(v.z), c3 = float_to_ikey(v.w);
+        if (c0 > kv[K - 1]) list_insert<K>(kv, ki, c0, col);
+        if (c1 > kv[K - 1]) list_insert<K>(kv, ki, c1, col + 1);
+        if (c2 > kv[K - 1]) list_insert<K>(kv, ki, c2, col + 2);
+        if (c3 > kv[K - 1]) list_insert<K>(kv, ki, c3, col + 3);
       }
     }
-    // merge the parts of a row: the lower part keeps its entries ahead of equal ones from higher columns
+    for (int r = 0; r < k; ++r) {
+      const uint64_t head = ((uint64_t)((uint32_t)kv[0] ^ 0x80000000u) << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)ki[0]);
+      uint64_t top = head;
 #pragma unroll
-    for (int d = 1; d < TPR; d <<= 1) {
-      int ok[K], oi[K];
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        ok[j] = __shfl_xor_sync(0xFFFFFFFFu, kv[j], d);
-        oi[j] = __shfl_xor_sync(0xFFFFFFFFu, ki[j], d);
+      for (int d = 1; d < L; d <<= 1) {
+        const uint64_t o = __shfl_xor_sync(FULL, top, d);
+        top = o > top ? o : top;
       }
-      if ((part & d) == 0) {
+      if (head == top && kv[0] != (int)0x80000000) {   // entries differ in their columns: one lane
+        cand[r] = top;
 #pragma unroll
-        for (int j = 0; j < K; ++j) list_insert<K>(kv, ki, ok[j], oi[j]);
+        for (int j = 0; j + 1 < K; ++j) { kv[j] = kv[j + 1]; ki[j] = ki[j + 1]; }
+        kv[K - 1] = (int)0x80000000;
       }
     }
-    // full-row softmax denominator for the conventions that normalise over all N
-    float rowsum = 0.f;
-    const float vmax = ikey_to_float(TPR == 1 ? kv[0] : __shfl_sync(0xFFFFFFFFu, kv[0], (tid & 31) - part));
-    if (mode != MOE_TOPK_MODE_B) {
-      if (active)
-        for (int v = v_lo; v < v_hi; ++v) {
-          const float4 x = *reinterpret_cast<const float4*>(rowp + v * 4);
-          rowsum += expf(x.x - vmax) + expf(x.y - vmax) + expf(x.z - vmax) + expf(x.w - vmax);
-        }
+  }
+  __syncwarp();
+
+  // ---- softmax over the k selected (mode B) or against the whole row (modes A)
+  const float vmax = key_to_float((uint32_t)(cand[0] >> 32));
+  constexpr int RL = (K + L - 1) / L;
+  float e[RL];
+  uint32_t ec[RL];
+  float denom = 0.f;
 #pragma unroll
-      for (int d = 1; d < TPR; d <<= 1) rowsum += __shfl_xor_sync(0xFFFFFFFFu, rowsum, d);
+  for (int t = 0; t < RL; ++t) {
+    const int r = t * L + sub;
+    e[t] = 0.f; ec[t] = 0u;
+    if (r < k) {
+      const uint64_t ent = cand[r];
+      e[t] = expf(key_to_float((uint32_t)(ent >> 32)) - vmax);
+      ec[t] = 0xFFFFFFFFu - (uint32_t)ent;
     }
-    if (active && part == 0) {
-      float e[K];
-      float denom = 0.f;
+    denom += e[t];
+  }
+  if (mode != MOE_TOPK_MODE_B) {
+    denom = 0.f;
 #pragma unroll
-      for (int j = 0; j < K; ++j) {
-        e[j] = j < k ? expf(ikey_to_float(kv[j]) - vmax) : 0.f;
-        denom += e[j];
-      }
-      if (mode != MOE_TOPK_MODE_B) denom = rowsum;
-      float renorm = 0.f;
+    for (int i = 0; i < EPT / 4; ++i)
+      denom += (expf(x[4 * i] - vmax) + expf(x[4 * i + 1] - vmax)) + (expf(x[4 * i + 2] - vmax) + expf(x[4 * i + 3] - vmax));
+  }
 #pragma unroll
-      for (int j = 0; j < K; ++j) { e[j] = e[j] / denom; renorm += e[j]; }
-      const int64_t o = (row0 + row_in_tile) * (int64_t)k;
+  for (int d = 1; d < L; d <<= 1) denom += __shfl_xor_sync(FULL, denom, d);
+  float renorm = 0.f;
 #pragma unroll
-      for (int j = 0; j < K; ++j) {
-        if (j < k) {
-          scores[o + j] = mode == MOE_TOPK_MODE_A_RENORM ? e[j] / renorm : e[j];
-          if (idx64) idx64[o + j] = (int64_t)ki[j];
-          if (idx32) idx32[o + j] = (int32_t)ki[j];
-        }
-      }
+  for (int t = 0; t < RL; ++t) { e[t] = e[t] / denom; renorm += e[t]; }
+  if (mode == MOE_TOPK_MODE_A_RENORM) {
+#pragma unroll
+    for (int d = 1; d < L; d <<= 1) renorm += __shfl_xor_sync(FULL, renorm, d);
+#pragma unroll
+    for (int t = 0; t < RL; ++t) e[t] = e[t] / renorm;
+  }
+  if (!live) return;
+  const int64_t o = row * (int64_t)k;
+#pragma unroll
+  for (int t = 0; t < RL; ++t) {
+    const int r = t * L + sub;
+    if (r < k) {
+      scores[o + r] = e[t];
+      if (idx64) idx64[o + r] = (int64_t)ec[t];
+      if (idx32) idx32[o + r] = (int32_t)ec[t];
     }
   }
 }
 
-template <int K, int TPR>
-static int launch_tile(const float* logits, int64_t M, int N, int64_t ld, int k, int mode, float* scores,
+template <int K, int L, int EPT>
+static int launch_group(const float* logits, int64_t M, int N, int64_t ld, int k, int mode, float* scores,
+                        int64_t* idx64, int32_t* idx32, cudaStream_t st) {
+  const int64_t blocks = ceil_div64(M, GROUP_WARPS * (32 / L));     // M * 8 fits an int: so does this
+  topk_group_kernel<K, L, EPT><<<(unsigned)blocks, GROUP_WARPS * 32, 0, st>>>(logits, M, N, ld, k, mode, scores, idx64, idx32);
+  MOE_CHECK_LAUNCH("topk_group_kernel");
+  return MOE_OK;
+}
+
+// ------------------------------------------------------------------------------------
+// lane-per-row kernel: many rows of at most 32 logits, small k (k <= 8, N % 4 == 0, 16-byte aligned rows)
+//
+// With so few logits a row is one lane's work: a warp stages 32 rows in its own part of shared memory with 16-byte
+// cp.async (coalesced, the only read of the logits), every lane takes V, the K-th largest of the maxima of 16 pairs of
+// neighbouring logits (two sorted lists of eight) - a lower bound of the K-th largest logit - and passes the logits not
+// below V (NaNs are not; they do not enter V either) in column order through a sorted list of K entries.  Scores and
+// indices leave through shared memory as contiguous runs of the warp's 32 rows.
+//
+// What bounds it: the stores and the lists.  Measured (us, thread-per-row tiles before -> now): 1048576 x 16, k = 2:
+// 63 -> 30; 1048576 x 8: 59 -> 27; 16384 x 16: 3.6 -> 2.5.  (The same form for 128 logits: 132 us for 1048576 rows
+// against 140 with four lanes per row, but twice its time on tied logits, and 6.7 against 4.9 us for 16384 rows: not built.)
+// ------------------------------------------------------------------------------------
+constexpr int LANE_WARPS = 4;
+constexpr int LANE_NMAX = 32;
+
+__device__ __forceinline__ void sort8_desc(float (&a)[16], int o) {   // 19 exchanges
+  ce_desc(a[o + 0], a[o + 2]); ce_desc(a[o + 1], a[o + 3]); ce_desc(a[o + 4], a[o + 6]); ce_desc(a[o + 5], a[o + 7]);
+  ce_desc(a[o + 0], a[o + 4]); ce_desc(a[o + 1], a[o + 5]); ce_desc(a[o + 2], a[o + 6]); ce_desc(a[o + 3], a[o + 7]);
+  ce_desc(a[o + 0], a[o + 1]); ce_desc(a[o + 2], a[o + 3]); ce_desc(a[o + 4], a[o + 5]); ce_desc(a[o + 6], a[o + 7]);
+  ce_desc(a[o + 2], a[o + 4]); ce_desc(a[o + 3], a[o + 5]);
+  ce_desc(a[o + 1], a[o + 4]); ce_desc(a[o + 3], a[o + 6]);
+  ce_desc(a[o + 1], a[o + 2]); ce_desc(a[o + 3], a[o + 4]); ce_desc(a[o + 5], a[o + 6]);
+}
+
+template <int K>
+__global__ void __launch_bounds__(LANE_WARPS * 32)
+topk_lane_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld, int k, int mode,
+                 float* __restrict__ scores, int64_t* __restrict__ idx64, int32_t* __restrict__ idx32) {
+  constexpr int NV = LANE_NMAX / 4;
+  __shared__ __align__(16) float lane_s[LANE_WARPS][32 * (LANE_NMAX + 4)];   // rows; later 32 x k scores and columns
+  static_assert(32 * 8 * 2 <= 32 * (LANE_NMAX + 4), "the output of 32 rows fits where their logits were");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pitch = N + 4;                           // floats: rows stay 16-byte aligned and spread over the banks
+  float* buf = lane_s[warp];
+  const float* mine = buf + lane * pitch;
+  const int nv = N >> 2;
+  const int rpi = 32 / nv, lr = lane / nv, lc = lane - lr * nv;   // staging: rows per instruction, this lane's row and vector
+  const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(buf) + (uint32_t)(lr * pitch + lc * 4) * 4u;
+  const float NEG_INF = __int_as_float((int)0xFF800000);
+  const int64_t n_tiles = (M + 31) / 32;
+
+  for (int64_t tile = (int64_t)blockIdx.x * LANE_WARPS + warp; tile < n_tiles; tile += (int64_t)gridDim.x * LANE_WARPS) {
+    const int64_t row0 = tile * 32;
+    const int rows = (int)(M - row0 < 32 ? M - row0 : 32);
+    __syncwarp();                                    // the previous tile's output has left the buffer
+    if (lr < rpi) {
+      const float* src = logits + (row0 + lr) * ld + lc * 4;
+      uint32_t dst = dst0;
+      for (int r = lr; r < rows; r += rpi) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+        src += rpi * ld;
+        dst += (uint32_t)(rpi * pitch) * 4u;
+      }
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+
+    float x[LANE_NMAX], g[16];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      float4 f = make_float4(NEG_INF, NEG_INF, NEG_INF, NEG_INF);
+      if (v < nv) f = *reinterpret_cast<const float4*>(mine + v * 4);
+      x[4 * v] = f.x; x[4 * v + 1] = f.y; x[4 * v + 2] = f.z; x[4 * v + 3] = f.w;
+      g[2 * v] = fmaxf(NEG_INF, fmaxf(f.x, f.y));
+      g[2 * v + 1] = fmaxf(NEG_INF, fmaxf(f.z, f.w));
+    }
+    sort8_desc(g, 0);
+    sort8_desc(g, 8);
+    float V = fmaxf(g[K - 1], g[8 + K - 1]);
+#pragma unroll
+    for (int i = 1; i < K; ++i) V = fmaxf(V, fminf(g[i - 1], g[8 + K - i - 1]));
+
+    uint32_t m = 0u;
+#pragma unroll
+    for (int b = 0; b < LANE_NMAX; ++b) m |= !(x[b] < V) ? (1u << b) : 0u;
+    m &= N < 32 ? (1u << N) - 1u : 0xFFFFFFFFu;
+    if (lane >= rows) m = 0u;                        // lanes past the last row worked on whatever the buffer held
+
+    int kv[K], ki[K];                                // equal keys: the earlier column stays ahead
+#pragma unroll
+    for (int j = 0; j < K; ++j) { kv[j] = (int)0x80000000; ki[j] = 0; }
+    while (m) {
+      const int col = __ffs(m) - 1;
+      m &= m - 1u;
+      list_insert<K>(kv, ki, float_to_ikey(mine[col]), col);
+    }
+
+    // softmax over the k selected (mode B) or against the whole row (modes A)
+    const float vmax = ikey_to_float(kv[0]);
+    float e[K];
+    float denom = 0.f;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      e[j] = j < k ? expf(ikey_to_float(kv[j]) - vmax) : 0.f;
+      denom += e[j];
+    }
+    if (mode != MOE_TOPK_MODE_B) {                   // columns past N hold -inf: they add nothing
+      denom = 0.f;
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        if (v < nv)
+          denom += (expf(x[4 * v] - vmax) + expf(x[4 * v + 1] - vmax)) + (expf(x[4 * v + 2] - vmax) + expf(x[4 * v + 3] - vmax));
+    }
+    float renorm = 0.f;
+#pragma unroll
+    for (int j = 0; j < K; ++j) { e[j] = e[j] / denom; renorm += e[j]; }
+    if (mode == MOE_TOPK_MODE_A_RENORM) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) e[j] = e[j] / renorm;
+    }
+
+    __syncwarp();                                    // every lane is done with its logits
+    int* col_s = reinterpret_cast<int*>(buf) + 32 * k;
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+      if (j < k) { buf[lane * k + j] = e[j]; col_s[lane * k + j] = ki[j]; }
+    __syncwarp();
+    const int64_t o = row0 * (int64_t)k;
+    for (int i = lane; i < rows * k; i += 32) {
+      scores[o + i] = buf[i];
+      const int c = col_s[i];
+      if (idx64) idx64[o + i] = (int64_t)c;
+      if (idx32) idx32[o + i] = (int32_t)c;
+    }
+  }
+}
+
+template <int K>
+static int launch_lane(const float* logits, int64_t M, int N, int64_t ld, int k, int mode, float* scores,
                        int64_t* idx64, int32_t* idx32, int sm_count, cudaStream_t st) {
-  const int rows_per_tile = TILE_THREADS / TPR;
-  const size_t smem = (size_t)rows_per_tile * (N + 4) * sizeof(float);
-  if (smem > 48 * 1024)   // per device, cheap: set on every such launch
-    MOE_CUDA_CHECK(cudaFuncSetAttribute(topk_tile_kernel<K, TPR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024));
-  int64_t blocks = ceil_div64(M, rows_per_tile);
-  const int64_t cap = (int64_t)sm_count * 3;
-  if (blocks > cap) blocks = cap;
-  topk_tile_kernel<K, TPR><<<(unsigned)blocks, TILE_THREADS, smem, st>>>(logits, M, N, ld, k, mode, rows_per_tile, scores,
-                                                                        idx64, idx32);
-  MOE_CHECK_LAUNCH("topk_tile_kernel");
+  int64_t blocks = ceil_div64(M, 32 * LANE_WARPS);
+  if (blocks > (int64_t)sm_count * 8) blocks = (int64_t)sm_count * 8;
+  topk_lane_kernel<K><<<(unsigned)blocks, LANE_WARPS * 32, 0, st>>>(logits, M, N, ld, k, mode, scores, idx64, idx32);
+  MOE_CHECK_LAUNCH("topk_lane_kernel");
   return MOE_OK;
 }
 
@@ -731,22 +949,37 @@ extern "C" int moe_topk_softmax(const float* logits, int64_t M, int64_t N, int64
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int n = (int)N;
-  if (n <= 1024 && k <= 8 && n >= 8 && (n % 4 == 0) && (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0) &&
-      M >= 2048) {
-    // enough rows to give every SM a tile; below that the warp-per-row kernel has the shorter critical path
-    // thread-per-row tiles: TPR threads share a row so that a tile is always <= 128 x 128 floats
-    const int tpr = n <= 128 ? 1 : (n <= 256 ? 2 : (n <= 512 ? 4 : 8));
-#define MOE_TILE_CASE(K_, T_) return launch_tile<K_, T_>(logits, M, n, ld, k, mode, scores, indices, indices32, dev.sm_count, st)
-#define MOE_TILE_K(K_) { if (tpr == 1) MOE_TILE_CASE(K_, 1); if (tpr == 2) MOE_TILE_CASE(K_, 2); if (tpr == 4) MOE_TILE_CASE(K_, 4); MOE_TILE_CASE(K_, 8); }
-    if (k <= 2) MOE_TILE_K(2)
-    if (k <= 4) MOE_TILE_K(4)
-    if (k <= 6) MOE_TILE_K(6)
-    MOE_TILE_K(8)
-#undef MOE_TILE_K
-#undef MOE_TILE_CASE
+  const bool vec_rows = (n % 4 == 0) && (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
+  // Measured (us): 320 rows of 128, k = 6: a warp per row 2.5, lane groups 3.5; of 256, k = 8: 3.2, 3.3; of 512: 4.0, 3.3;
+  // of 1024: 5.8, 3.4.  2048 rows of 16: a lane per row 2.5, lane groups 2.5; 8192: 2.6, 2.6; 32768: 2.9, 3.8; rows of 64
+  // (a lane per row is built for 32 at most): 32768 4.3, 4.5.
+  if (n <= 1024 && k <= 8 && n >= 8 && vec_rows && (M >= 2048 || n > 256)) {
+    if (n <= LANE_NMAX) {
+#define MOE_LANE_CASE(K_) return launch_lane<K_>(logits, M, n, ld, k, mode, scores, indices, indices32, dev.sm_count, st)
+      if (k <= 2) MOE_LANE_CASE(2);
+      if (k <= 4) MOE_LANE_CASE(4);
+      if (k <= 6) MOE_LANE_CASE(6);
+      MOE_LANE_CASE(8);
+#undef MOE_LANE_CASE
+    }
+#define MOE_GROUP_CASE(K_, L_, E_) return launch_group<K_, L_, E_>(logits, M, n, ld, k, mode, scores, indices, indices32, st)
+#define MOE_GROUP_K(K_)                          \
+  {                                              \
+    if (n <= 64) MOE_GROUP_CASE(K_, 4, 16);      \
+    if (n <= 128) MOE_GROUP_CASE(K_, 4, 32);     \
+    if (n <= 256) MOE_GROUP_CASE(K_, 8, 32);     \
+    if (n <= 512) MOE_GROUP_CASE(K_, 16, 32);    \
+    MOE_GROUP_CASE(K_, 32, 32);                  \
+  }
+    if (k <= 2) MOE_GROUP_K(2)
+    if (k <= 4) MOE_GROUP_K(4)
+    if (k <= 6) MOE_GROUP_K(6)
+    MOE_GROUP_K(8)
+#undef MOE_GROUP_K
+#undef MOE_GROUP_CASE
   }
   if (n <= 1024 && k <= 64) {
-    const bool vec = (n % 4 == 0) && (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
+    const bool vec = vec_rows;
 #define MOE_WARP_CASE(E_, V_) return launch_warp<E_, V_>(logits, M, n, ld, k, mode, scores, indices, indices32, dev.sm_count, st)
     if (n <= 32) MOE_WARP_CASE(1, 1);
     if (n <= 64) MOE_WARP_CASE(2, 1);
