@@ -214,6 +214,17 @@ int moe_router_topk_splitk(const void* x, const void* Wr, int64_t T, int H, int 
                            float* scores, int64_t* indices, int32_t* indices32, float* logits_out, void* ws,
                            size_t ws_bytes, int32_t* status, void* stream);
 
+/* ---- expert GEMM of un-sorted rows in one call -----------------------------------------
+ * Y[(t,s),:] = X[t,:] . W[ids[t,s]]^T: grouped_gemm(X, W, expert_indices) (kernels/grouped_gemm_tilelang.py:859-895)
+ * as one C call that enqueues moe_route_histogram, moe_gather_rows where H % 64 != 0, and the grouped GEMM.
+ *   X [T,H], W [E,I,H], Y [T*k,I], 16-bit of `dtype`; ids [T,k] int64 (ids_int64 = 1) or int32.
+ *   ws: moe_grouped_gemm_routed_workspace(T,k,H,E) bytes of device scratch, 256-byte aligned.
+ * Same results and the same refusals as the calls one by one; scratch is the caller's, nothing is kept.
+ */
+size_t moe_grouped_gemm_routed_workspace(int64_t T, int k, int H, int E);
+int moe_grouped_gemm_routed(const void* X, int64_t T, int k, const void* ids, int ids_int64, const void* W, void* Y, int H,
+                            int I, int E, int dtype, void* ws, size_t ws_bytes, int32_t* status, void* stream);
+
 /* ---- the whole layer in one call -----------------------------------------------------
  * FusedMoEPyTorch.forward / FusedMoETileLang.forward (kernels/fusedmoe_baseline.py:46-91,
  * kernels/fusedmoe_tilelang.py:309-417) as one C call that sequences the entry points above on

@@ -42,6 +42,8 @@ SIGNATURES = {
     "moe_debug_bounds_status": (_i32, [C.POINTER(C.c_int32), _vp]),
     "moe_grouped_gemm_peer_scatter": (_i32, [_vp, _vp, _vp, _vp, _vp, C.POINTER(C.c_void_p), _i32, _i64, _i64, _i64,
                                              _i32, _i32, _i32, _i32, _vp, _vp]),
+    "moe_grouped_gemm_routed_workspace": (_sz, [_i64, _i32, _i32, _i32]),
+    "moe_grouped_gemm_routed": (_i32, [_vp, _i64, _i32, _vp, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _sz, _vp, _vp]),
     "moe_layer_workspace": (_sz, [_i64, _i32, _i32, _i32, _i32, _i32]),
     "moe_layer_forward": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _i32, _i32,
                                  _vp, _sz, _vp, _vp, _vp, _vp]),

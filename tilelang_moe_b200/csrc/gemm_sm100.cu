@@ -129,6 +129,7 @@ struct Params {
   int l2_hints = 0;        // 128-row kernel: 0 none, 1 evict-first for weights read once, 2 + evict-last for shared weights
   int mixed = 0;           // 128-row kernel: single-tile and multi-tile experts interleaved in the tile order
   int m64 = 0;             // 128-row kernel: tiles with at most 64 live rows as M = 64 instructions
+  int pdl = 0;             // host side: launched behind another kernel of the same call
   int64_t y_rows = 0;      // rows of Y when dst_rows scatters into it (the checked build compares every destination with it)
 };
 
@@ -464,6 +465,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
     tmem_relinquish();
   }
+  pdl_wait();
+  pdl_trigger();
   for (int e = threadIdx.x; e <= E; e += blockDim.x) offs[e] = p.offsets ? p.offsets[e] : (e == 0 ? 0 : p.dense_rows);
   __syncthreads();
   if (warp == 2) { if (mixed) mixed_prefix(tstart, lstart, offs, E, lane); else tile_prefix(tstart, offs, E, TILE_ROWS, lane); }
@@ -1293,8 +1296,8 @@ static int launch_g(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensor
   static std::atomic<bool> attr_set[64];
   int rc = allow_dynamic_smem(grouped_gemm_kernel<MT, BN, EPI, GATHER>, SMEM, attr_set);
   if (rc) return rc;
-  grouped_gemm_kernel<MT, BN, EPI, GATHER><<<grid, GATHER ? NUM_THREADS_GATHER : NUM_THREADS, SMEM, st>>>(tA, tB, tB2, p);
-  MOE_CHECK_LAUNCH("grouped_gemm_kernel");
+  MOE_LAUNCH("grouped_gemm_kernel", grouped_gemm_kernel<MT, BN, EPI, GATHER>, (unsigned)grid,
+             GATHER ? NUM_THREADS_GATHER : NUM_THREADS, SMEM, st, p.pdl != 0, tA, tB, tB2, p);
   return MOE_OK;
 }
 template <int MT, int BN, int EPI>
@@ -1326,6 +1329,7 @@ struct GatherArgs {           // A rows fetched through an index list instead of
   int64_t src_rows = 0;
   int64_t dense_rows = 0;     // > 0 with offsets == nullptr: one group of this many rows (E must be 1)
   int w_slots = 0;            // see Params::w_slots
+  bool pdl = false;           // behind another kernel of the same library call
 };
 
 static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const void* B2, const int32_t* offsets,
@@ -1334,11 +1338,34 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
                              void* const* peer_base, int n_peers, int64_t expected_rows, int dtype,
                              const GatherArgs& ga = GatherArgs());
 
+int moe::grouped_gemm_ex(int epilogue, const void* A, const void* B, const void* B2, const int32_t* offsets,
+                         const int32_t* dst_rows, const float* row_w, void* Y, int64_t ldy, int64_t max_rows,
+                         int64_t expected_rows, int K, int N, int E, int dtype, int32_t* status, void* stream, bool pdl) {
+  GatherArgs ga;
+  ga.pdl = pdl;
+  return grouped_gemm_impl(epilogue, A, B, B2, offsets, dst_rows, row_w, Y, ldy, max_rows, K, N, E, status, stream,
+                           nullptr, nullptr, 0, expected_rows, dtype, ga);
+}
+
 extern "C" int moe_grouped_gemm(int epilogue, const void* A, const void* B, const void* B2, const int32_t* offsets,
                                 const int32_t* dst_rows, const float* row_w, void* Y, int64_t ldy, int64_t max_rows,
                                 int64_t expected_rows, int K, int N, int E, int dtype, int32_t* status, void* stream) {
-  return grouped_gemm_impl(epilogue, A, B, B2, offsets, dst_rows, row_w, Y, ldy, max_rows, K, N, E, status, stream,
-                           nullptr, nullptr, 0, expected_rows, dtype);
+  return moe::grouped_gemm_ex(epilogue, A, B, B2, offsets, dst_rows, row_w, Y, ldy, max_rows, expected_rows, K, N, E, dtype,
+                              status, stream, false);
+}
+
+int moe::grouped_gemm_gathered_ex(int epilogue, const void* X, int64_t x_rows, const int32_t* gather_idx, int gather_div,
+                                  const void* B, const void* B2, const int32_t* offsets, const int32_t* dst_rows,
+                                  const float* row_w, void* Y, int64_t ldy, int64_t max_rows, int64_t expected_rows, int K,
+                                  int N, int E, int dtype, int32_t* status, void* stream, bool pdl) {
+  if (!gather_idx) return fail(MOE_ERR_ARG, "grouped_gemm_gathered: null index list");
+  if (gather_div < 1 || x_rows < 1 || x_rows > 0x7FFFFFFFll)
+    return fail(MOE_ERR_ARG, "grouped_gemm_gathered: bad gather_div=%d or x_rows=%lld", gather_div, (long long)x_rows);
+  if (K % 64) return fail(MOE_ERR_UNSUPPORTED, "grouped_gemm_gathered: K=%d must be a multiple of 64", K);
+  GatherArgs ga;
+  ga.idx = gather_idx; ga.div = gather_div; ga.src_rows = x_rows; ga.pdl = pdl;
+  return grouped_gemm_impl(epilogue, X, B, B2, offsets, dst_rows, row_w, Y, ldy, max_rows, K, N, E, status, stream,
+                           nullptr, nullptr, 0, expected_rows, dtype, ga);
 }
 
 extern "C" int moe_grouped_gemm_gathered(int epilogue, const void* X, int64_t x_rows, const int32_t* gather_idx,
@@ -1346,15 +1373,8 @@ extern "C" int moe_grouped_gemm_gathered(int epilogue, const void* X, int64_t x_
                                          const int32_t* dst_rows, const float* row_w, void* Y, int64_t ldy,
                                          int64_t max_rows, int64_t expected_rows, int K, int N, int E, int dtype,
                                          int32_t* status, void* stream) {
-  using namespace moe;
-  if (!gather_idx) return fail(MOE_ERR_ARG, "grouped_gemm_gathered: null index list");
-  if (gather_div < 1 || x_rows < 1 || x_rows > 0x7FFFFFFFll)
-    return fail(MOE_ERR_ARG, "grouped_gemm_gathered: bad gather_div=%d or x_rows=%lld", gather_div, (long long)x_rows);
-  if (K % 64) return fail(MOE_ERR_UNSUPPORTED, "grouped_gemm_gathered: K=%d must be a multiple of 64", K);
-  GatherArgs ga;
-  ga.idx = gather_idx; ga.div = gather_div; ga.src_rows = x_rows;
-  return grouped_gemm_impl(epilogue, X, B, B2, offsets, dst_rows, row_w, Y, ldy, max_rows, K, N, E, status, stream,
-                           nullptr, nullptr, 0, expected_rows, dtype, ga);
+  return moe::grouped_gemm_gathered_ex(epilogue, X, x_rows, gather_idx, gather_div, B, B2, offsets, dst_rows, row_w, Y, ldy,
+                                       max_rows, expected_rows, K, N, E, dtype, status, stream, false);
 }
 
 // Router GEMM with the top-k + softmax of every logits row done in the epilogue (declared in common.cuh; the
@@ -1402,9 +1422,10 @@ int moe::router_topk_gemm(const void* x, const void* Wr, int64_t T, int H, int E
 
 int moe::grouped_gemm_scatter_slots(const void* A, const void* B, const int32_t* offsets, const int32_t* dst_rows,
                                     const float* row_w, int w_slots, void* Y, int64_t ldy, int64_t max_rows, int K, int N,
-                                    int E, int dtype, int32_t* status, void* stream) {
+                                    int E, int dtype, int32_t* status, void* stream, bool pdl) {
   GatherArgs ga;
   ga.w_slots = w_slots;
+  ga.pdl = pdl;
   return grouped_gemm_impl(MOE_GEMM_SCALE_SCATTER_DSTW, A, B, nullptr, offsets, dst_rows, row_w, Y, ldy, max_rows, K, N, E,
                            status, stream, nullptr, nullptr, 0, 0, dtype, ga);
 }
@@ -1533,6 +1554,7 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
   for (int g = 0; g < 16; ++g) p.peer_base[g] = (peer_base && g < n_peers) ? peer_base[g] : nullptr;
   p.w_by_dst = w_by_dst;
   p.w_slots = ga.w_slots;
+  p.pdl = ga.pdl;
   p.y_rows = max_rows;     // a scatter permutes the sorted rows: the output has as many rows as the sorted input
   p.dense_rows = (int)ga.dense_rows;
   p.a_gather = ga.idx; p.a_src = A; p.a_div = ga.div; p.a_src_rows = (int)ga.src_rows; p.a_rows = (int)max_rows;

@@ -52,6 +52,27 @@ static LayerScratch layer_layout(int64_t T, int k, int H, int I, int E, int SI) 
   return L;
 }
 
+// Overlapping a kernel's start with the end of the one before it hides a few us per boundary, whatever the size; the
+// kernels of a long batch last a hundred times that, and CTAs that wait beside them only take their room.
+constexpr int64_t PDL_MAX_TOKENS = 4096;
+
+struct RoutedScratch {
+  size_t counts, offsets, perm, hist, xs, total;
+};
+static RoutedScratch routed_layout(int64_t T, int k, int H, int E) {
+  RoutedScratch L;
+  const size_t n = (size_t)T * k;
+  size_t o = 0;
+  auto take = [&](size_t bytes) { const size_t at = o; o += align256(bytes); return at; };
+  L.counts = take((size_t)E * 4);
+  L.offsets = take((size_t)(E + 1) * 4);
+  L.perm = take(n * 4);
+  L.hist = take(moe_route_histogram_workspace((int64_t)n, E));
+  L.xs = take(H % 64 == 0 ? 0 : n * (size_t)H * 2);
+  L.total = o;
+  return L;
+}
+
 // two events per device for the fork / join around the shared expert; created once, never destroyed
 static int layer_events(cudaEvent_t* fork, cudaEvent_t* join) {
   static cudaEvent_t ev[64][2];
@@ -72,6 +93,37 @@ static int layer_events(cudaEvent_t* fork, cudaEvent_t* join) {
 }
 
 }  // namespace moe
+
+extern "C" size_t moe_grouped_gemm_routed_workspace(int64_t T, int k, int H, int E) {
+  if (T < 0 || k < 0 || H < 1 || E < 1) return 0;
+  return moe::routed_layout(T, k, H, E).total;
+}
+
+extern "C" int moe_grouped_gemm_routed(const void* X, int64_t T, int k, const void* ids, int ids_int64, const void* W, void* Y,
+                                       int H, int I, int E, int dtype, void* ws, size_t ws_bytes, int32_t* status,
+                                       void* stream) {
+  using namespace moe;
+  if (T < 0 || k < 0 || H < 1 || E < 1)
+    return fail(MOE_ERR_ARG, "grouped_gemm_routed: bad shape T=%lld k=%d H=%d E=%d", (long long)T, k, H, E);
+  if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255)) return fail(MOE_ERR_ARG, "grouped_gemm_routed: workspace must be 256-byte aligned");
+  const RoutedScratch L = routed_layout(T, k, H, E);
+  if (ws_bytes < L.total) return fail(MOE_ERR_WORKSPACE, "grouped_gemm_routed: workspace %zu < %zu", ws_bytes, L.total);
+  unsigned char* base = reinterpret_cast<unsigned char*>(ws);
+  int32_t* counts = reinterpret_cast<int32_t*>(base + L.counts);
+  int32_t* offsets = reinterpret_cast<int32_t*>(base + L.offsets);
+  int32_t* perm = reinterpret_cast<int32_t*>(base + L.perm);
+  const int64_t n = T * k;
+  int rc = route_histogram_ex(ids, ids_int64, n, E, nullptr, counts, offsets, perm, nullptr, base + L.hist,
+                              moe_route_histogram_workspace(n, E), status, stream, 0, false);
+  if (rc) return rc;
+  if (H % 64 == 0)     // the GEMM fetches the rows of X through the permutation itself
+    return grouped_gemm_gathered_ex(MOE_GEMM_PLAIN, X, T, perm, k, W, nullptr, offsets, perm, nullptr, Y, I, n, 0, H, I, E, dtype,
+                                    status, stream, true);
+  rc = moe_gather_rows(X, perm, k, n, H, base + L.xs, nullptr, nullptr, stream);
+  if (rc) return rc;
+  return grouped_gemm_ex(MOE_GEMM_PLAIN, base + L.xs, W, nullptr, offsets, perm, nullptr, Y, I, n, 0, H, I, E, dtype, status,
+                         stream, true);
+}
 
 extern "C" size_t moe_layer_workspace(int64_t T, int k, int H, int I, int E, int SI) {
   if (T < 1 || k < 1 || H < 1 || I < 1 || E < 1 || SI < 0) return 0;
@@ -102,6 +154,7 @@ extern "C" int moe_layer_forward(const void* x, const void* router_weight, const
   void* act = base + L.act;
   void* yk = base + L.yk;
   const int64_t n = T * k;
+  const bool pdl = T <= PDL_MAX_TOKENS;
   int rc;
   // once the side stream has been forked, every return - also an error - first makes `stream` wait for it again:
   // inside a stream capture an unjoined fork would turn the caller's end-of-capture into an unrelated failure
@@ -171,24 +224,24 @@ routed:
     // k + 1 entries per token: the k routed ones from idx32 and a virtual one for expert E; five launches in all
     const int64_t n1 = T * (k + 1);
     rc = route_histogram_ex(idx32, 0, n1, E + 1, nullptr, counts, offsets, perm, nullptr, base + L.hist,
-                            moe_route_histogram_workspace(n1, E + 1), status, stream, k);
+                            moe_route_histogram_workspace(n1, E + 1), status, stream, k, pdl);
     if (rc) return rc;
-    rc = moe_grouped_gemm_gathered(MOE_GEMM_SILU_GATE, x, T, perm, k + 1, routed_gate, routed_up, offsets, nullptr, nullptr, act,
-                                   I, n1, 0, H, I, E + 1, dtype, status, stream);
+    rc = grouped_gemm_gathered_ex(MOE_GEMM_SILU_GATE, x, T, perm, k + 1, routed_gate, routed_up, offsets, nullptr, nullptr, act,
+                                   I, n1, 0, H, I, E + 1, dtype, status, stream, pdl);
     if (rc) return rc;
-    rc = grouped_gemm_scatter_slots(act, routed_down, offsets, perm, scores, k, yk, H, n1, I, H, E + 1, dtype, status, stream);
+    rc = grouped_gemm_scatter_slots(act, routed_down, offsets, perm, scores, k, yk, H, n1, I, H, E + 1, dtype, status, stream, pdl);
     if (rc) return rc;
-    return moe_combine(yk, nullptr, nullptr, nullptr, T, k + 1, H, dtype, out, stream);
+    return combine_ex(yk, nullptr, nullptr, nullptr, T, k + 1, H, dtype, out, stream, pdl);
   }
-  rc = moe_route_histogram(idx32, 0, n, E, nullptr, counts, offsets, perm, nullptr, base + L.hist,
-                           moe_route_histogram_workspace(n, E), status, stream);
+  rc = route_histogram_ex(idx32, 0, n, E, nullptr, counts, offsets, perm, nullptr, base + L.hist,
+                          moe_route_histogram_workspace(n, E), status, stream, 0, pdl);
   if (rc) return leave(rc);
   if (H % 64 == 0) {
-    rc = moe_grouped_gemm_gathered(MOE_GEMM_SILU_GATE, x, T, perm, k, routed_gate, routed_up, offsets, nullptr, nullptr, act, I,
-                                   n, 0, H, I, E, dtype, status, stream);
+    rc = grouped_gemm_gathered_ex(MOE_GEMM_SILU_GATE, x, T, perm, k, routed_gate, routed_up, offsets, nullptr, nullptr, act, I,
+                                  n, 0, H, I, E, dtype, status, stream, pdl);
     if (rc) return leave(rc);
-    rc = moe_grouped_gemm(MOE_GEMM_SCALE_SCATTER_DSTW, act, routed_down, nullptr, offsets, perm, scores, yk, H, n, 0, I, H, E,
-                          dtype, status, stream);
+    rc = grouped_gemm_ex(MOE_GEMM_SCALE_SCATTER_DSTW, act, routed_down, nullptr, offsets, perm, scores, yk, H, n, 0, I, H, E,
+                         dtype, status, stream, pdl);
     if (rc) return leave(rc);
   } else {
     float* wsorted = reinterpret_cast<float*>(base + L.wsorted);
@@ -201,10 +254,11 @@ routed:
                           dtype, status, stream);
     if (rc) return leave(rc);
   }
+  const bool joined = forked;
   if (forked) {   // join: the combine reads the shared expert's output
     MOE_CUDA_CHECK(cudaEventRecord(ev_join, reinterpret_cast<cudaStream_t>(side_stream)));
     MOE_CUDA_CHECK(cudaStreamWaitEvent(st, ev_join, 0));
     forked = false;
   }
-  return moe_combine(yk, shared_out, nullptr, nullptr, T, k, H, dtype, out, stream);
+  return combine_ex(yk, shared_out, nullptr, nullptr, T, k, H, dtype, out, stream, pdl && !joined);
 }

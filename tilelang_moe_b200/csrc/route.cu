@@ -56,6 +56,8 @@ template <int UNIT>
 __global__ void __launch_bounds__(RWPB * 32)
 route_count_kernel(const void* __restrict__ ids, int is64, int64_t n, int E, const int32_t* __restrict__ id_map,
                    int32_t* __restrict__ unit_counts, int32_t* __restrict__ status, int kx) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ int32_t sh[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int32_t* wh = sh + (size_t)w * E;
@@ -86,6 +88,8 @@ route_count_kernel(const void* __restrict__ ids, int is64, int64_t n, int E, con
 __global__ void __launch_bounds__(1024)
 route_scan_kernel(int32_t* __restrict__ unit_counts, int64_t n_units, int E, int32_t* __restrict__ counts,
                   int32_t* __restrict__ offsets) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ int32_t warp_tot[32];
   __shared__ int32_t carry_s;
   __shared__ int32_t part[1024];     // [P][Ec]: entries of expert e in the p-th share of the units
@@ -146,6 +150,8 @@ template <int UNIT>
 __global__ void __launch_bounds__(RWPB * 32)
 route_scatter_kernel(const void* __restrict__ ids, int is64, int64_t n, int E, const int32_t* __restrict__ id_map,
                      const int32_t* __restrict__ unit_base, int32_t* __restrict__ perm, int32_t* __restrict__ inv, int kx) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ int32_t sh[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -200,6 +206,8 @@ route_small_kernel(const void* __restrict__ ids, int is64, int n, int E, const i
   const unsigned lt_mask = (1u << lane) - 1u;
   for (int i = tid; i < 33 * E; i += 1024) sh[i] = 0;
   if (tid == 0) carry_s = 0;
+  pdl_wait();
+  pdl_trigger();
   __syncthreads();
   // a thread owns entries tid, tid + 1024, ...: at most RSINGLE_MAX / 1024 of them, kept in registers for the
   // permutation rounds below (the loads are independent, so they are all in flight together)
@@ -267,6 +275,8 @@ __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ perm, int div, int64_t n_rows,
                    int vec_per_row, uint4* __restrict__ dst, const float* __restrict__ w_src,
                    float* __restrict__ w_dst) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t)gridDim.x * 8;
   for (int64_t p = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); p < n_rows; p += nwarps) {
@@ -327,6 +337,8 @@ template <bool F16>
 __global__ void __launch_bounds__(256)
 combine_kernel(const uint4* __restrict__ Yk, const uint4* __restrict__ shared, const int32_t* __restrict__ row_of,
                const float* __restrict__ scale, int64_t T, int k, int vec_per_row, uint4* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t total = T * vec_per_row;
   for (int64_t g = (int64_t)blockIdx.x * 256 + threadIdx.x; g < total; g += (int64_t)gridDim.x * 256) {
     const int64_t t = g / vec_per_row;
@@ -374,6 +386,8 @@ __global__ void __launch_bounds__(256)
 router_logits_kernel(const uint4* __restrict__ x, const uint4* __restrict__ Wr, int64_t T, int vec_per_row, int E,
                      float* __restrict__ logits, int k, int mode, float* __restrict__ scores,
                      int64_t* __restrict__ idx64, int32_t* __restrict__ idx32) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ uint4 wsh[];   // [E][vec_per_row]
   const int lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < E * vec_per_row; i += 256) wsh[i] = __ldg(Wr + i);
@@ -548,14 +562,14 @@ extern "C" int moe_route_histogram(const void* topk_idx, int idx_is_int64, int64
                                    int32_t* counts, int32_t* offsets, int32_t* perm, int32_t* inv, void* ws,
                                    size_t ws_bytes, int32_t* status, void* stream) {
   return moe::route_histogram_ex(topk_idx, idx_is_int64, n, E, id_map, counts, offsets, perm, inv, ws, ws_bytes, status,
-                                 stream, 0);
+                                 stream, 0, false);
 }
 
 // kx > 0: n counts a virtual list in which every kx stored ids are followed by one entry of expert E - 1 (declared in
 // common.cuh; used by the single-call layer to run the shared expert as one more group of the routed GEMMs)
 int moe::route_histogram_ex(const void* topk_idx, int idx_is_int64, int64_t n, int E, const int32_t* id_map,
                             int32_t* counts, int32_t* offsets, int32_t* perm, int32_t* inv, void* ws, size_t ws_bytes,
-                            int32_t* status, void* stream, int kx) {
+                            int32_t* status, void* stream, int kx, bool pdl) {
   using namespace moe;
   if (n < 0 || E < 1) return fail(MOE_ERR_ARG, "route_histogram: bad size n=%lld E=%d", (long long)n, E);
   if (!counts || !offsets) return fail(MOE_ERR_ARG, "route_histogram: null counts/offsets");
@@ -580,8 +594,8 @@ int moe::route_histogram_ex(const void* topk_idx, int idx_is_int64, int64_t n, i
     const size_t smem1 = (size_t)33 * E * 4;
     if (smem1 > 48 * 1024)
       MOE_CUDA_CHECK(cudaFuncSetAttribute(route_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
-    route_small_kernel<<<1, 1024, smem1, st>>>(topk_idx, idx_is_int64, (int)n, E, id_map, counts, offsets, perm, inv, status, kx);
-    MOE_CHECK_LAUNCH("route_small_kernel");
+    MOE_LAUNCH("route_small_kernel", route_small_kernel, 1u, 1024u, smem1, st, pdl, topk_idx, idx_is_int64, (int)n, E, id_map,
+               counts, offsets, perm, inv, status, kx);
     return MOE_OK;
   }
   const int64_t units = ceil_div64(n, small ? RUNIT_SMALL : RUNIT);
@@ -594,18 +608,13 @@ int moe::route_histogram_ex(const void* topk_idx, int idx_is_int64, int64_t n, i
     MOE_CUDA_CHECK(cudaFuncSetAttribute(route_scatter_kernel<RUNIT_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
   const unsigned blocks = (unsigned)ceil_div64(units, RWPB);
-  if (units > 0) {
-    if (small) route_count_kernel<RUNIT_SMALL><<<blocks, RWPB * 32, smem, st>>>(topk_idx, idx_is_int64, n, E, id_map, unit_counts, status, kx);
-    else route_count_kernel<RUNIT><<<blocks, RWPB * 32, smem, st>>>(topk_idx, idx_is_int64, n, E, id_map, unit_counts, status, kx);
-    MOE_CHECK_LAUNCH("route_count_kernel");
-  }
-  route_scan_kernel<<<1, 1024, 0, st>>>(unit_counts, units, E, counts, offsets);
-  MOE_CHECK_LAUNCH("route_scan_kernel");
-  if (units > 0 && (perm || inv)) {
-    if (small) route_scatter_kernel<RUNIT_SMALL><<<blocks, RWPB * 32, smem, st>>>(topk_idx, idx_is_int64, n, E, id_map, unit_counts, perm, inv, kx);
-    else route_scatter_kernel<RUNIT><<<blocks, RWPB * 32, smem, st>>>(topk_idx, idx_is_int64, n, E, id_map, unit_counts, perm, inv, kx);
-    MOE_CHECK_LAUNCH("route_scatter_kernel");
-  }
+  if (units > 0)
+    MOE_LAUNCH("route_count_kernel", small ? route_count_kernel<RUNIT_SMALL> : route_count_kernel<RUNIT>, blocks, RWPB * 32u, smem,
+               st, pdl, topk_idx, idx_is_int64, n, E, id_map, unit_counts, status, kx);
+  MOE_LAUNCH("route_scan_kernel", route_scan_kernel, 1u, 1024u, 0, st, units > 0 || pdl, unit_counts, units, E, counts, offsets);
+  if (units > 0 && (perm || inv))
+    MOE_LAUNCH("route_scatter_kernel", small ? route_scatter_kernel<RUNIT_SMALL> : route_scatter_kernel<RUNIT>, blocks, RWPB * 32u,
+               smem, st, true, topk_idx, idx_is_int64, n, E, id_map, unit_counts, perm, inv, kx);
   return MOE_OK;
 }
 
@@ -632,7 +641,11 @@ extern "C" int moe_gather_rows(const void* src, const int32_t* perm, int div, in
 
 extern "C" int moe_combine(const void* Yk, const void* shared, const int32_t* row_of, const float* scale, int64_t T,
                            int k, int64_t H, int dtype, void* out, void* stream) {
-  using namespace moe;
+  return moe::combine_ex(Yk, shared, row_of, scale, T, k, H, dtype, out, stream, false);
+}
+
+int moe::combine_ex(const void* Yk, const void* shared, const int32_t* row_of, const float* scale, int64_t T, int k, int64_t H,
+                    int dtype, void* out, void* stream, bool pdl) {
   if (dtype != MOE_DTYPE_BF16 && dtype != MOE_DTYPE_F16) return fail(MOE_ERR_ARG, "combine: unknown dtype %d", dtype);
   if (T < 0 || k < 0 || H < 8 || H % 8) return fail(MOE_ERR_ARG, "combine: bad shape T=%lld k=%d H=%lld", (long long)T, k, (long long)H);
   if (T == 0) return MOE_OK;
@@ -646,15 +659,9 @@ extern "C" int moe_combine(const void* Yk, const void* shared, const int32_t* ro
   int64_t blocks = ceil_div64(total, 256);
   const int64_t cap = (int64_t)dev.sm_count * 8;
   if (blocks > cap) blocks = cap;
-  if (dtype == MOE_DTYPE_F16)
-    combine_kernel<true><<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const uint4*>(Yk), reinterpret_cast<const uint4*>(shared), row_of, scale, T, k, (int)(H / 8),
-        reinterpret_cast<uint4*>(out));
-  else
-    combine_kernel<false><<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const uint4*>(Yk), reinterpret_cast<const uint4*>(shared), row_of, scale, T, k, (int)(H / 8),
-        reinterpret_cast<uint4*>(out));
-  MOE_CHECK_LAUNCH("combine_kernel");
+  MOE_LAUNCH("combine_kernel", dtype == MOE_DTYPE_F16 ? combine_kernel<true> : combine_kernel<false>, (unsigned)blocks, 256u, 0,
+             reinterpret_cast<cudaStream_t>(stream), pdl, reinterpret_cast<const uint4*>(Yk), reinterpret_cast<const uint4*>(shared),
+             row_of, scale, T, k, (int)(H / 8), reinterpret_cast<uint4*>(out));
   return MOE_OK;
 }
 
@@ -732,6 +739,8 @@ __global__ void __launch_bounds__(256)
 router_reduce_topk_kernel(const float* __restrict__ part, int S, int64_t T, int E, int k, int mode,
                           float* __restrict__ scores, int64_t* __restrict__ idx64, int32_t* __restrict__ idx32,
                           float* __restrict__ logits_out) {
+  pdl_wait();
+  pdl_trigger();
   const unsigned FULL = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t)gridDim.x * 8;
@@ -822,9 +831,9 @@ extern "C" int moe_router_topk_splitk(const void* x, const void* Wr, int64_t T, 
   if (rc) return rc;
   int64_t blocks = ceil_div64(T, 8);
   if (blocks > (int64_t)dev.sm_count * 8) blocks = (int64_t)dev.sm_count * 8;
-  router_reduce_topk_kernel<<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const float*>(ws), S, T, E, k, mode, scores, indices, indices32, logits_out);
-  MOE_CHECK_LAUNCH("router_reduce_topk_kernel");
+  MOE_LAUNCH("router_reduce_topk_kernel", router_reduce_topk_kernel, (unsigned)blocks, 256u, 0,
+             reinterpret_cast<cudaStream_t>(stream), true, reinterpret_cast<const float*>(ws), S, T, E, k, mode, scores, indices,
+             indices32, logits_out);
   return MOE_OK;
 }
 

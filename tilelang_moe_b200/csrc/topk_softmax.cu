@@ -37,6 +37,7 @@ template <int ELTS, int VEC>
 __global__ void __launch_bounds__(128)
 topk_warp_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld, int k, int mode,
                  float* __restrict__ scores, int64_t* __restrict__ idx64, int32_t* __restrict__ idx32) {
+  pdl_trigger();
   const unsigned FULL = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t)gridDim.x * 4;
@@ -189,6 +190,7 @@ topk_group_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane & (L - 1), rw = lane / L;
   const int64_t row0 = ((int64_t)blockIdx.x * GROUP_WARPS + warp) * RPW;
+  pdl_trigger();
   if (row0 >= M) return;                            // whole warps only: no block barrier below
   const int64_t row = row0 + rw;
   const bool live = row < M;
@@ -450,6 +452,7 @@ __global__ void __launch_bounds__(LANE_WARPS * 32)
 topk_lane_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld, int k, int mode,
                  float* __restrict__ scores, int64_t* __restrict__ idx64, int32_t* __restrict__ idx32) {
   constexpr int NV = LANE_NMAX / 4;
+  pdl_trigger();
   __shared__ __align__(16) float lane_s[LANE_WARPS][32 * (LANE_NMAX + 4)];   // rows; later 32 x k scores and columns
   static_assert(32 * 8 * 2 <= 32 * (LANE_NMAX + 4), "the output of 32 rows fits where their logits were");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -666,6 +669,7 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
                   int slice, int vec_ok, float* __restrict__ scores, int64_t* __restrict__ idx64,
                   int32_t* __restrict__ idx32, int32_t* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_trigger();
   const unsigned FULL = 0xFFFFFFFFu;
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned C = cluster.num_blocks();

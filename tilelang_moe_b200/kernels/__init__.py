@@ -82,15 +82,7 @@ def grouped_gemm(X: torch.Tensor, W: torch.Tensor, expert_indices: torch.Tensor,
         raise ValueError("expert_indices must be (total_tokens,) or (total_tokens, k)")
     E, I, H = W.shape
     k = expert_indices.shape[1] if expert_indices.dim() == 2 else 1
-    n = X.shape[0] * k
-    _, offsets, perm, _ = _ops.route_histogram(expert_indices, E, want_inv=False)
-    Y = torch.empty(n, I, dtype=X.dtype, device=X.device)
-    if H % 64 == 0:     # the GEMM fetches the rows of X through the permutation itself
-        _ops.grouped_gemm_sorted(_ops.GEMM_PLAIN, X.contiguous(), W.contiguous(), offsets, dst_rows=perm, out=Y,
-                                 gather=perm, gather_div=k)
-    else:
-        xs = _ops.gather_rows(X.contiguous(), perm, div=k)
-        _ops.grouped_gemm_sorted(_ops.GEMM_PLAIN, xs, W.contiguous(), offsets, dst_rows=perm, out=Y)
+    Y = _ops.grouped_gemm_routed(X.contiguous(), W.contiguous(), expert_indices, k)
     return Y.view(X.shape[0], k, I) if expert_indices.dim() == 2 else Y
 
 

@@ -214,6 +214,33 @@ def grouped_gemm_sorted(epilogue: int, A: torch.Tensor, B: torch.Tensor, offsets
     return out
 
 
+def grouped_gemm_routed(X: torch.Tensor, W: torch.Tensor, ids: torch.Tensor, k: int) -> torch.Tensor:
+    """Y [T*k, I] = rows of X [T, H] times their experts' W [E, I, H], expert ids [T] or [T, k] (int64 / int32): routing
+    tables and GEMM in one library call on one scratch buffer."""
+    _need_cuda(ids, X, W)
+    dt = _dtype_code(X, W)
+    if ids.dtype not in (torch.int64, torch.int32):
+        raise ValueError("expert ids must be int64 or int32")
+    if X.dim() != 2 or W.dim() != 3 or not X.is_contiguous() or not W.is_contiguous():
+        raise ValueError("X must be contiguous [rows,K], W contiguous [E,N,K]")
+    T, H = X.shape
+    E, I, K2 = W.shape
+    if K2 != H:
+        raise ValueError(f"inner dimensions differ: X has K={H}, W has K={K2}")
+    ids = ids.contiguous()
+    dev = X.device
+    lib = _lib.load()
+    need = lib.moe_grouped_gemm_routed_workspace(T, k, H, E)
+    ws = torch.empty(max(need, 4), dtype=torch.uint8, device=dev)
+    Y = torch.empty(T * k, I, dtype=X.dtype, device=dev)
+    with torch.cuda.device(dev):
+        rc = lib.moe_grouped_gemm_routed(_ptr(X), T, k, _ptr(ids), int(ids.dtype == torch.int64), _ptr(W), _ptr(Y), H, I, E, dt,
+                                         _ptr(ws), need, _ptr(status_buffer(dev)), _stream())
+    _lib.check(rc, "moe_grouped_gemm_routed")
+    _after(dev)
+    return Y
+
+
 def combine(Yk: torch.Tensor, k: int, shared: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
             row_of: Optional[torch.Tensor] = None, scale: Optional[torch.Tensor] = None,
             T: Optional[int] = None) -> torch.Tensor:
