@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from oracle import moe_oracle as O
 from tilelang_moe_b200 import kernels, ops
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +43,30 @@ def test_grouped_gemm_in_one_call(cuda, lib, T, k, H, I, E, dtype):
     torch.cuda.synchronize()
     assert torch.equal(out, want.flip(0))
     ops.check_status(cuda)
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 136, 8), (127, 256, 8), (128, 160, 6), (129, 256, 1), (255, 256, 8), (256, 200, 3),
+                                   (257, 256, 8), (38000, 256, 8), (300, 128, 8), (300, 104, 8)])
+@pytest.mark.parametrize("kind", ["normal", "equal", "sorted"])
+def test_router_selection_in_the_epilogue(cuda, lib, T, E, k, kind):
+    """One-kernel router: CTA pairs above 128 experts, single CTAs up to there; few logits above the bound (normal), all of
+    them equal to it, and more above it than a row may park (ascending logits)."""
+    H = 128
+    g = torch.Generator().manual_seed(T + E)
+    X = (torch.round(torch.randn(T, H, generator=g) * 4) / 4).bfloat16()
+    W = (torch.round(torch.randn(E, H, generator=g) * 4) / 8).bfloat16()
+    if kind == "equal":
+        W = W[:1].repeat(E, 1)
+    elif kind == "sorted":
+        X[:, 0] = 8.0
+        W.zero_()
+        W[:, 0] = torch.arange(E).float() / 4
+    X, W = X.to(cuda), W.to(cuda)
+    lg = torch.full((T, E), float("nan"), device=cuda)
+    for mode in ("B", "A", "A_renorm"):
+        s, i = ops.router_topk_softmax(X, W, k, mode=mode, logits_out=lg, fused=True)
+        ops.check_status(cuda)
+        assert torch.equal(lg, ops.router_logits(X, W))
+        s_ref, i_ref = O.topk_softmax(lg.cpu(), k, mode)
+        assert torch.equal(i.cpu(), i_ref)
+        torch.testing.assert_close(s.cpu(), s_ref, rtol=1e-6, atol=1e-30)

@@ -84,7 +84,8 @@ struct Cfg {
   static constexpr int TABLE_OFFSET = BAR_OFFSET + 256;
   static constexpr int STAGING_OFFSET = (TABLE_OFFSET + 3 * (MAX_E + 1) * 4 + 127) & ~127;   // 16-byte accesses
   static constexpr int SMEM_BYTES = STAGING_OFFSET + 1024;  // + alignment slack
-  // peer epilogue: 4 warps x 32 rows x (128 B + 16 B pad) to turn per-thread rows into 128-byte row segments
+  // peer epilogue: 4 warps x 32 rows x (128 B + 16 B pad) to turn per-thread rows into 128-byte row segments;
+  // router epilogue: 4 warps x 32 rows x ROUTER_CAP parked logits
   static constexpr int STAGING_PITCH = 144;
   static constexpr int SMEM_BYTES_PEER = SMEM_BYTES + 4 * 32 * STAGING_PITCH;
   static_assert(STAGING_OFFSET % 16 == 0 && STAGING_PITCH % 16 == 0, "staging rows are accessed as 16-byte vectors");
@@ -420,6 +421,131 @@ __device__ __forceinline__ uint32_t pack_out(float a, float b, int f16) {
 // 341 rows per expert 41 -> 20 us.
 __device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 
+// One row of router logits per thread, N of them (N % 8 == 0, at most 256) in tensor-memory columns taddr ...: top-k,
+// softmax and the three stores.
+//
+// A sorted list fed with every logit costs an insertion for nearly every column, because one of the warp's 32 rows wants
+// it: about 11 thousand instructions per tile, and with one tile per CTA nothing hides them.  Instead the first pass
+// keeps only the eight largest of the maxima of eight neighbouring columns; the k-th of them, V, is a lower bound of the
+// k-th largest logit.  The second pass parks the logits not below V in shared memory (NaNs are not; they do not enter V
+// either) and adds up the softmax denominator; those, a dozen as a rule, go through the list in column order.  A warp
+// with more than ROUTER_CAP of them in one row feeds the list from tensor memory after all.
+constexpr int ROUTER_CAP = 16;
+__device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t taddr, int grow, bool row_ok,
+                                                    unsigned char* park, int lane) {
+  constexpr int KMAX = 8;
+  const int chunks = (p.N + 31) / 32;
+  const float NEG_INF = __int_as_float((int)0xFF800000);
+  float s[KMAX];
+#pragma unroll
+  for (int j = 0; j < KMAX; ++j) s[j] = NEG_INF;
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    uint32_t v[32];
+    tmem_ld32(taddr + c * 32, v);
+    tmem_ld_wait();
+    float g[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float m = NEG_INF;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) m = fmaxf(m, __uint_as_float(v[8 * q + j]));
+      g[q] = c * 32 + q * 8 < p.N ? m : NEG_INF;
+    }
+    auto ce = [](float& x, float& y) { const float hi = fmaxf(x, y), lo = fminf(x, y); x = hi; y = lo; };
+    ce(g[0], g[1]); ce(g[2], g[3]); ce(g[0], g[2]); ce(g[1], g[3]); ce(g[1], g[2]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[4 + i] = fmaxf(s[4 + i], g[3 - i]);   // the eight largest of both lists, bitonic
+#pragma unroll
+    for (int st = KMAX / 2; st > 0; st >>= 1)
+#pragma unroll
+      for (int i = 0; i < KMAX; ++i)
+        if ((i & st) == 0) ce(s[i], s[i | st]);
+    if (p.r_logits && row_ok) {
+      float* dst = p.r_logits + (int64_t)grow * p.N + c * 32;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (c * 32 + j * 4 < p.N)   // N % 8 == 0: whole 16-byte vectors
+          *reinterpret_cast<uint4*>(dst + j * 4) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    }
+  }
+  float V = s[0];
+#pragma unroll
+  for (int j = 1; j < KMAX; ++j) V = j < p.r_k ? s[j] : V;
+  const float top = s[0];
+
+  float2* mine = reinterpret_cast<float2*>(park) + lane;      // entry j of this row at mine[32 * j]
+  int cnt = 0;
+  double total = 0.0;                      // 32-term fp32 sums added up in fp64: the denominator of up to 256 terms
+#pragma unroll 1                            // keeps the scores within 1e-6 of an exactly summed softmax
+  for (int c = 0; c < chunks; ++c) {
+    uint32_t v[32];
+    tmem_ld32(taddr + c * 32, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const float x = __uint_as_float(v[j]);
+      if (!(x < V) && c * 32 + (j & ~7) < p.N) {
+        if (cnt < ROUTER_CAP) mine[32 * cnt] = make_float2(x, __int_as_float(c * 32 + j));
+        ++cnt;
+      }
+    }
+    if (p.r_mode != MOE_TOPK_MODE_B) {      // the conventions that normalise over all experts
+      float part = 0.f;
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (c * 32 + j < p.N) part += expf(__uint_as_float(v[j]) - top);
+      total += (double)part;
+    }
+  }
+  int kv[KMAX], ki[KMAX];
+#pragma unroll
+  for (int j = 0; j < KMAX; ++j) { kv[j] = (int)0x80000000; ki[j] = 0; }
+  if (!__any_sync(0xFFFFFFFFu, cnt > ROUTER_CAP)) {
+    for (int j = 0; j < cnt; ++j) {         // ascending columns and a strict comparison: lowest index first among equals
+      const float2 e = mine[32 * j];
+      list_insert<KMAX>(kv, ki, float_to_ikey(e.x), __float_as_int(e.y));
+    }
+    __syncwarp();                           // tensor-memory loads below and in the next tile are warp-wide
+  } else {
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+      uint32_t v[32];
+      tmem_ld32(taddr + c * 32, v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const int col = c * 32 + j;
+        const int key = float_to_ikey(__uint_as_float(v[j]));
+        if (col < p.N && key > kv[KMAX - 1]) list_insert<KMAX>(kv, ki, key, col);
+      }
+    }
+  }
+  const float vmax = ikey_to_float(kv[0]);
+  if (row_ok) {
+    float e[KMAX];
+    float denom = 0.f;
+#pragma unroll
+    for (int j = 0; j < KMAX; ++j) {
+      e[j] = j < p.r_k ? expf(ikey_to_float(kv[j]) - vmax) : 0.f;
+      denom += e[j];
+    }
+    if (p.r_mode != MOE_TOPK_MODE_B) denom = (float)total;
+    float renorm = 0.f;
+#pragma unroll
+    for (int j = 0; j < KMAX; ++j) { e[j] = e[j] / denom; renorm += e[j]; }
+    const int64_t o = (int64_t)grow * p.r_k;
+#pragma unroll
+    for (int j = 0; j < KMAX; ++j) {
+      if (j < p.r_k) {
+        p.r_scores[o + j] = p.r_mode == MOE_TOPK_MODE_A_RENORM ? e[j] / renorm : e[j];
+        if (p.r_idx64) p.r_idx64[o + j] = (int64_t)ki[j];
+        if (p.r_idx32) p.r_idx32[o + j] = (int32_t)ki[j];
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------ kernel
 template <int MT, int BN, int EPI, bool GATHER>
 __global__ void __launch_bounds__(GATHER ? NUM_THREADS_GATHER : NUM_THREADS, 1)
@@ -669,71 +795,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * MT * BN + half * BN);
       if (EPI == EPI_ROUTER) {
-        // This thread's accumulator row holds the N logits of one token: keep the k largest in a sorted list
-        // (ascending column scan + strict comparison = lowest index first among equals), then normalise.
-        constexpr int KMAX = 8;
-        int kv[KMAX], ki[KMAX];
-#pragma unroll
-        for (int j = 0; j < KMAX; ++j) { kv[j] = (int)0x80000000; ki[j] = 0; }
-        const int chunks = (p.N + 31) / 32;
-#pragma unroll 1
-        for (int c = 0; c < chunks; ++c) {
-          uint32_t v[32];
-          tmem_ld32(taddr + c * 32, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int col = c * 32 + j;
-            const int key = float_to_ikey(__uint_as_float(v[j]));
-            if (col < p.N && key > kv[KMAX - 1]) list_insert<KMAX>(kv, ki, key, col);
-          }
-          if (p.r_logits && row_ok) {
-            float* dst = p.r_logits + (int64_t)grow * p.N + c * 32;
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (c * 32 + j * 4 < p.N)   // N % 8 == 0: whole 16-byte vectors
-                *reinterpret_cast<uint4*>(dst + j * 4) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          }
-        }
-        const float vmax = ikey_to_float(kv[0]);
-        float rowsum = 0.f;
-        if (p.r_mode != MOE_TOPK_MODE_B) {       // conventions that normalise over all experts: second pass over TMEM
-          double total = 0.0;                    // 32-term fp32 sums added up in fp64: the denominator of up to 256 terms
-#pragma unroll 1                                  // keeps the scores within 1e-6 of an exactly summed softmax
-          for (int c = 0; c < chunks; ++c) {
-            uint32_t v[32];
-            tmem_ld32(taddr + c * 32, v);
-            tmem_ld_wait();
-            float part = 0.f;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (c * 32 + j < p.N) part += expf(__uint_as_float(v[j]) - vmax);
-            total += (double)part;
-          }
-          rowsum = (float)total;
-        }
-        if (row_ok) {
-          float e[KMAX];
-          float denom = 0.f;
-#pragma unroll
-          for (int j = 0; j < KMAX; ++j) {
-            e[j] = j < p.r_k ? expf(ikey_to_float(kv[j]) - vmax) : 0.f;
-            denom += e[j];
-          }
-          if (p.r_mode != MOE_TOPK_MODE_B) denom = rowsum;
-          float renorm = 0.f;
-#pragma unroll
-          for (int j = 0; j < KMAX; ++j) { e[j] = e[j] / denom; renorm += e[j]; }
-          const int64_t o = (int64_t)grow * p.r_k;
-#pragma unroll
-          for (int j = 0; j < KMAX; ++j) {
-            if (j < p.r_k) {
-              p.r_scores[o + j] = p.r_mode == MOE_TOPK_MODE_A_RENORM ? e[j] / renorm : e[j];
-              if (p.r_idx64) p.r_idx64[o + j] = (int64_t)ki[j];
-              if (p.r_idx32) p.r_idx32[o + j] = (int32_t)ki[j];
-            }
-          }
-        }
+        router_row_epilogue(p, taddr, grow, row_ok, smem + C::STAGING_OFFSET + (warp - 2) * 32 * C::STAGING_PITCH, lane);
       } else {
 #pragma unroll 1
       for (int c = 0; c < OUT_COLS / 32; ++c) {
@@ -1022,7 +1084,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     bool ok = true;
     for (int tile = cluster_id; ok && tile < total_tiles; tile += n_clusters) {
       const Tile t = decode_tile(tile, tstart, offs, E, NT, TILE_ROWS);
-      const bool light = t.row_end - t.row0 <= BM;           // 128-row tile: 64 rows per CTA
+      const bool light = EPI != EPI_ROUTER && t.row_end - t.row0 <= BM;           // 128-row tile: 64 rows per CTA
       const int n0 = t.n_tile * OUT_COLS;
       const int a_row = t.row0 + (int)rank * (light ? BM / 2 : BM);
       const uint32_t tx = light ? 2u * (C::A_BYTES / 2 + C::B_BYTES) : 2u * C::STAGE_BYTES;
@@ -1122,7 +1184,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     bool ok = true;
     for (int tile = cluster_id; ok && tile < total_tiles; tile += n_clusters) {
       const Tile t = decode_tile(tile, tstart, offs, E, NT, TILE_ROWS);
-      const bool light = t.row_end - t.row0 <= BM;
+      const bool light = EPI != EPI_ROUTER && t.row_end - t.row0 <= BM;
       if (!mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag, p.status, 14)) { ok = false; break; }
       tc_fence_after();
       // 256-row tile: lane = row of this CTA's 128; 128-row tile: lanes 0..63 and 64..127 both hold this CTA's 64 rows,
@@ -1154,7 +1216,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         if (EPI == EPI_PEER) ybase = p.peer_base[p.row_rank[grow]];
       }
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-      if (GATE) {
+      if (EPI == EPI_ROUTER) {
+        router_row_epilogue(p, taddr, grow, row_ok, smem + C::STAGING_OFFSET + (warp - 2) * 32 * C::STAGING_PITCH, lane);
+      } else if (GATE) {
         // accumulator columns: [gate 64 | up 64] per group of 64 output columns; a 256-row tile holds two groups,
         // a 128-row tile one per lane half
         const int groups = light ? 1 : 2;
@@ -1292,7 +1356,7 @@ template <int MT, int BN, int EPI, bool GATHER>
 static int launch_g(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2, const Params& p, int grid,
                     cudaStream_t st) {
   using C = Cfg<MT, BN>;
-  constexpr int SMEM = EPI == EPI_PEER ? C::SMEM_BYTES_PEER : C::SMEM_BYTES;
+  constexpr int SMEM = EPI == EPI_PEER || EPI == EPI_ROUTER ? C::SMEM_BYTES_PEER : C::SMEM_BYTES;
   static std::atomic<bool> attr_set[64];
   int rc = allow_dynamic_smem(grouped_gemm_kernel<MT, BN, EPI, GATHER>, SMEM, attr_set);
   if (rc) return rc;
@@ -1311,7 +1375,7 @@ static int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMa
 template <int EPI>
 static int launch_pair(const CUtensorMap& tA, const CUtensorMap& tA64, const CUtensorMap& tB, const CUtensorMap& tB2,
                        const Params& p, int grid, cudaStream_t st) {
-  constexpr int SMEM = EPI == EPI_PEER ? PairCfg::SMEM_BYTES_PEER : PairCfg::SMEM_BYTES;
+  constexpr int SMEM = EPI == EPI_PEER || EPI == EPI_ROUTER ? PairCfg::SMEM_BYTES_PEER : PairCfg::SMEM_BYTES;
   static std::atomic<bool> attr_set[64];
   int rc = allow_dynamic_smem(grouped_gemm_pair_kernel<EPI>, SMEM, attr_set);
   if (rc) return rc;
@@ -1397,7 +1461,6 @@ int moe::router_topk_gemm(const void* x, const void* Wr, int64_t T, int H, int E
   int rc = current_device_info(&dev);
   if (rc) return rc;
   const int f16 = dtype == MOE_DTYPE_F16;
-  const int BN = E > 128 ? 256 : 128;
   Params p;
   p.K = H; p.N = E; p.E = 1;
   p.num_n_tiles = 1;
@@ -1410,13 +1473,24 @@ int moe::router_topk_gemm(const void* x, const void* Wr, int64_t T, int H, int E
   CUtensorMap tA, tB;
   rc = make_tmap(&tA, x, (uint64_t)H, (uint64_t)T, 0, (uint32_t)BM, f16);
   if (rc) return rc;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (E > 128) {
+    // Two CTAs per 256-row tile, each staging half of the weight rows: the weight comes out of L2 once per 256 tokens
+    // instead of once per 128 (every CTA reads all of it, 48 KB per 64 columns of K with its own rows, 32 KB here), and
+    // that traffic took as long as HBM's.
+    // Measured (us; 16384 tokens, H = 7168, E = 256, k = 8, mode A): single CTAs, a list fed with every logit 97; pairs and
+    // parked logits 82 (HBM 36; the tensor pipe of the 128 SMs that hold a tile 44).
+    rc = make_tmap(&tB, Wr, (uint64_t)H, (uint64_t)E, 1, 128u, f16);
+    if (rc) return rc;
+    const int64_t units = (T + 2 * BM - 1) / (2 * BM);
+    const int pgrid = (int)(2 * units < dev.sm_count ? 2 * units : dev.sm_count) & ~1;
+    return launch_pair<EPI_ROUTER>(tA, tA, tB, tB, p, pgrid, st);
+  }
   rc = make_tmap(&tB, Wr, (uint64_t)H, (uint64_t)E, 1, (uint32_t)E, f16);    // only the E weight rows are fetched
   if (rc) return rc;
   p.b_tx_bytes = E * BK * 2;
   const int64_t tiles = (T + BM - 1) / BM;
   const int grid = (int)(tiles < dev.sm_count ? tiles : dev.sm_count);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (BN == 256) return launch<1, 256, EPI_ROUTER>(tA, tB, tB, p, grid, st);
   return launch<1, 128, EPI_ROUTER>(tA, tB, tB, p, grid, st);
 }
 
