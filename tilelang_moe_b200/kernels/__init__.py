@@ -129,8 +129,9 @@ class FusedMoETileLang:
                 out[:E].copy_(routed)
                 out[E].copy_(shared.reshape(shape))
                 return out
-            self._stack = (stack(routed_gate, shared_gate, (I, H)), stack(routed_up, shared_up, (I, H)),
-                           stack(routed_down, shared_down, (H, I)))
+            g, u, d = (stack(routed_gate, shared_gate, (I, H)), stack(routed_up, shared_up, (I, H)),
+                       stack(routed_down, shared_down, (H, I)))
+            self._stack = (g[E], u[E], d[E], g[:E], u[:E], d[:E])       # the views every forward passes on
             self._stack_key = key
         return self._stack
 
@@ -140,10 +141,7 @@ class FusedMoETileLang:
         st = self._stacked(shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down) \
             if self.n_shared_experts else None
         if st is not None:
-            E = routed_gate.shape[0]
-            g, u, d = st
-            return _layer.moe_forward_single_call(x, router_weight, g[E], u[E], d[E], g[:E], u[:E], d[:E],
-                                                  self.n_experts_per_token, ws=self.ws, logits=logits)
+            return _layer.moe_forward_single_call(x, router_weight, *st, self.n_experts_per_token, ws=self.ws, logits=logits)
         return _layer.moe_forward_single_call(x, router_weight, shared_gate if self.n_shared_experts else None,
                                               shared_up, shared_down, routed_gate, routed_up, routed_down,
                                               self.n_experts_per_token, ws=self.ws, logits=logits)

@@ -215,7 +215,7 @@ def moe_forward_single_call(x: torch.Tensor, router_weight: Optional[torch.Tenso
     y = ws.out if out is None else out.view(T, H)
     side = _side_stream(dev) if SI > 0 else None
     p = ops._ptr
-    with torch.cuda.device(dev):
+    with ops._on(dev):
         rc = _lib.load().moe_layer_forward(
             p(x_flat), p(router_weight) if logits is None else None, p(logits), p(shared_gate), p(shared_up), p(shared_down),
             p(routed_gate), p(routed_up), p(routed_down), T, H, I, E, k, SI, ops.DTYPE_CODE[x.dtype],

@@ -8,6 +8,7 @@ read after every call when ``MOE_B200_DEBUG=1``.
 """
 from __future__ import annotations
 
+import contextlib
 import os
 from typing import Optional, Tuple
 
@@ -42,8 +43,18 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+_getdevice, _rawstream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+_HERE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """torch.cuda.device(device), without its cost of some 2 us where that device is the current one already."""
+    return _HERE if device.index == _getdevice() else torch.cuda.device(device)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (no Stream object is made for it)."""
+    return _rawstream(_getdevice())
 
 
 def _need_cuda(*ts: torch.Tensor) -> None:
@@ -53,7 +64,9 @@ def _need_cuda(*ts: torch.Tensor) -> None:
 
 
 def status_buffer(device: torch.device) -> torch.Tensor:
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
+    key = device.index if isinstance(device, torch.device) else torch.device(device).index
+    if key is None:
+        key = torch.cuda.current_device()
     buf = _status.get(key)
     if buf is None:
         buf = torch.zeros(4, dtype=torch.int32, device=torch.device("cuda", key))
@@ -98,7 +111,7 @@ def topk_softmax(logits: torch.Tensor, k: int, mode="B", index_dtype: torch.dtyp
     scores = torch.empty(M, k, dtype=torch.float32, device=logits.device)
     idx64 = torch.empty(M, k, dtype=torch.int64, device=logits.device) if index_dtype == torch.int64 else None
     idx32 = torch.empty(M, k, dtype=torch.int32, device=logits.device) if (also_int32 or idx64 is None) else None
-    with torch.cuda.device(logits.device):
+    with _on(logits.device):
         rc = lib.moe_topk_softmax(_ptr(logits), M, N, logits.stride(0), k, _MODES[mode], _ptr(scores), _ptr(idx64),
                                   _ptr(idx32), _ptr(status_buffer(logits.device)), _stream())
     _lib.check(rc, "moe_topk_softmax")
@@ -129,7 +142,7 @@ def route_histogram(topk_idx: torch.Tensor, n_experts: int, want_perm: bool = Tr
     need = lib.moe_route_histogram_workspace(n, n_experts)
     if workspace is None or workspace.numel() * workspace.element_size() < need:
         workspace = torch.empty(max(need, 4), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = lib.moe_route_histogram(_ptr(ids), int(ids.dtype == torch.int64), n, n_experts, _ptr(id_map), _ptr(counts),
                                      _ptr(offsets), _ptr(perm), _ptr(inv), _ptr(workspace),
                                      workspace.numel() * workspace.element_size(), _ptr(status_buffer(dev)), _stream())
@@ -154,7 +167,7 @@ def gather_rows(src: torch.Tensor, perm: Optional[torch.Tensor], div: int = 1, o
         w_src = w_src.contiguous().view(-1)
         if w_out is None:
             w_out = torch.empty(n, dtype=torch.float32, device=src.device)
-    with torch.cuda.device(src.device):
+    with _on(src.device):
         rc = _lib.load().moe_gather_rows(_ptr(src), _ptr(perm), div, n, cols, _ptr(out), _ptr(w_src), _ptr(w_out), _stream())
     _lib.check(rc, "moe_gather_rows")
     return (out, w_out) if w_src is not None else out
@@ -197,7 +210,7 @@ def grouped_gemm_sorted(epilogue: int, A: torch.Tensor, B: torch.Tensor, offsets
     if out is None:
         odt = torch.float32 if epilogue == GEMM_PLAIN_F32 else A.dtype
         out = torch.empty(rows if out_rows is None else out_rows, N, dtype=odt, device=A.device)
-    with torch.cuda.device(A.device):
+    with _on(A.device):
         if gather is not None:
             name = "moe_grouped_gemm_gathered"
             rc = _lib.load().moe_grouped_gemm_gathered(
@@ -233,7 +246,7 @@ def grouped_gemm_routed(X: torch.Tensor, W: torch.Tensor, ids: torch.Tensor, k: 
     need = lib.moe_grouped_gemm_routed_workspace(T, k, H, E)
     ws = torch.empty(max(need, 4), dtype=torch.uint8, device=dev)
     Y = torch.empty(T * k, I, dtype=X.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = lib.moe_grouped_gemm_routed(_ptr(X), T, k, _ptr(ids), int(ids.dtype == torch.int64), _ptr(W), _ptr(Y), H, I, E, dt,
                                          _ptr(ws), need, _ptr(status_buffer(dev)), _stream())
     _lib.check(rc, "moe_grouped_gemm_routed")
@@ -253,7 +266,7 @@ def combine(Yk: torch.Tensor, k: int, shared: Optional[torch.Tensor] = None, out
     dt = _dtype_code(Yk, shared)
     if out is None:
         out = torch.empty(T, H, dtype=Yk.dtype, device=Yk.device)
-    with torch.cuda.device(Yk.device):
+    with _on(Yk.device):
         rc = _lib.load().moe_combine(_ptr(Yk), _ptr(shared), _ptr(row_of), _ptr(scale), T, k, H, dt, _ptr(out), _stream())
     _lib.check(rc, "moe_combine")
     return out
@@ -287,7 +300,7 @@ def router_logits(x: torch.Tensor, router_weight: torch.Tensor, out: Optional[to
     small = E <= 32 and E * H * 2 <= 200 * 1024        # the whole router weight fits one CTA's shared memory
     if not small and E % 8 == 0 and T > 0:
         return grouped_gemm_sorted(GEMM_PLAIN_F32, x, router_weight.unsqueeze(0), _offsets_0_T(T, x.device), out=out)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = _lib.load().moe_router_logits(_ptr(x), _ptr(router_weight), T, H, E, dt, _ptr(out),
                                            _ptr(status_buffer(x.device)), _stream())
     _lib.check(rc, "moe_router_logits")
@@ -325,7 +338,7 @@ def _router_topk_splitk(x, router_weight, k, mode, index_dtype, logits_out):
     ws = torch.empty(max(need, 16), dtype=torch.uint8, device=x.device)
     scores = torch.empty(T, k, dtype=torch.float32, device=x.device)
     idx = torch.empty(T, k, dtype=index_dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = lib.moe_router_topk_splitk(_ptr(x), _ptr(router_weight), T, H, E, k, _MODES[mode], dt, _ptr(scores),
                                         _ptr(idx) if index_dtype == torch.int64 else None,
                                         _ptr(idx) if index_dtype == torch.int32 else None, _ptr(logits_out), _ptr(ws),
@@ -371,7 +384,7 @@ def router_topk_softmax(x: torch.Tensor, router_weight: torch.Tensor, k: int, mo
         raise ValueError("logits_out must be a contiguous fp32 [T,E] tensor")
     scores = torch.empty(T, k, dtype=torch.float32, device=x.device)
     idx = torch.empty(T, k, dtype=index_dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = _lib.load().moe_router_topk(_ptr(x), _ptr(router_weight), T, H, E, k, _MODES[mode], dt,
                                          _ptr(scores), _ptr(idx) if index_dtype == torch.int64 else None,
                                          _ptr(idx) if index_dtype == torch.int32 else None, _ptr(logits_out),
@@ -390,7 +403,7 @@ def mhc_split_weights(fn: torch.Tensor) -> torch.Tensor:
     fn = fn.contiguous()
     R, K = fn.shape
     fn3 = torch.empty(3 * R, K, dtype=torch.bfloat16, device=fn.device)
-    with torch.cuda.device(fn.device):
+    with _on(fn.device):
         rc = _lib.load().moe_mhc_split_weights(_ptr(fn), R, K, _ptr(fn3), _stream())
     _lib.check(rc, "moe_mhc_split_weights")
     return fn3
@@ -419,7 +432,7 @@ def mhc_pre(residual: torch.Tensor, fn3: torch.Tensor, hc_scale: torch.Tensor, h
     post = torch.empty(T, hc, 1, dtype=torch.float32, device=dev)
     comb = torch.empty(T, hc, hc, dtype=torch.float32, device=dev)
     layer_input = torch.empty(T, hidden, dtype=torch.bfloat16, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = lib.moe_mhc_pre(_ptr(residual), _ptr(fn3), _ptr(hc_scale.contiguous()), _ptr(hc_base.contiguous()), T, hc,
                              hidden, rms_eps, hc_pre_eps, hc_sinkhorn_eps, hc_post_mult_value, sinkhorn_repeat,
                              _ptr(workspace), workspace.numel() * workspace.element_size(), _ptr(post), _ptr(comb),
@@ -441,7 +454,7 @@ def mhc_post(x: torch.Tensor, residual: torch.Tensor, post_layer_mix: torch.Tens
     if post_layer_mix.dtype != torch.float32 or comb_res_mix.dtype != torch.float32:
         raise ValueError("mixing coefficients must be float32")
     out = torch.empty(T, hc, hidden, dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = _lib.load().moe_mhc_post(_ptr(x.contiguous()), _ptr(residual.contiguous()), _ptr(post_layer_mix.contiguous()),
                                       _ptr(comb_res_mix.contiguous()), T, hc, hidden, _ptr(out), _stream())
     _lib.check(rc, "moe_mhc_post")
@@ -455,7 +468,7 @@ def ep_regroup(recv_counts: torch.Tensor, n_recv_bound: int):
     dev = recv_counts.device
     offsets = torch.empty(El + 1, dtype=torch.int32, device=dev)
     src_row = torch.empty(max(n_recv_bound, 1), dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = _lib.load().moe_ep_regroup(_ptr(recv_counts.contiguous()), G, El, _ptr(offsets), _ptr(src_row), _stream())
     _lib.check(rc, "moe_ep_regroup")
     return offsets, src_row
@@ -478,7 +491,7 @@ def ep_plan(cnt_all: torch.Tensor, G: int, e_local: int, rank: int, cap_rows: in
         out["dst_base"] = torch.empty(G * e_local, dtype=torch.int32, device=dev)
         out["ret_rank"] = torch.empty(cap_rows, dtype=torch.int32, device=dev)
         out["ret_row"] = torch.empty(cap_rows, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = _lib.load().moe_ep_plan(_ptr(cnt_all), G, e_local, rank, _ptr(out["offsets"]), _ptr(out["dst_base"]),
                                      _ptr(out["ret_rank"]), _ptr(out["ret_row"]), _stream())
     _lib.check(rc, "moe_ep_plan")
@@ -493,7 +506,7 @@ def ep_dispatch(x: torch.Tensor, perm: torch.Tensor, idx32: torch.Tensor, id_map
     _need_cuda(x, perm)
     n = perm.numel()
     arr = peer_recv_ptrs if not isinstance(peer_recv_ptrs, (list, tuple)) else _ptr_array(peer_recv_ptrs)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = _lib.load().moe_ep_dispatch(_ptr(x), _ptr(perm), _ptr(idx32), _ptr(id_map), _ptr(offsets), _ptr(dst_base),
                                          k, e_local, slot_lo, e_local if slot_hi is None else slot_hi, n, x.shape[1],
                                          arr, len(arr), _stream())
@@ -509,7 +522,7 @@ def ep_unique(idx32: torch.Tensor, id_map: torch.Tensor, e_local: int, G: int, o
     if "urank" not in out or out["urank"].shape[0] != Tl:
         out["urank"] = torch.empty(Tl, G, dtype=torch.int32, device=idx32.device)
         out["ucount"] = torch.empty(G, dtype=torch.int32, device=idx32.device)
-    with torch.cuda.device(idx32.device):
+    with _on(idx32.device):
         rc = _lib.load().moe_ep_unique(_ptr(idx32), _ptr(id_map), Tl, k, e_local, G, _ptr(out["urank"]), _ptr(out["ucount"]),
                                        _stream())
     _lib.check(rc, "moe_ep_unique")
@@ -529,7 +542,7 @@ def ep_plan_dedup(cnt_all: torch.Tensor, G: int, e_local: int, rank: int, cap_ro
         out["ret_row"] = torch.empty(cap_rows, dtype=torch.int32, device=dev)
     if "u_base" not in out:
         out["u_base"] = torch.empty(G, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rc = _lib.load().moe_ep_plan_dedup(_ptr(cnt_all), G, e_local, rank, _ptr(out["offsets"]), _ptr(out["dst_base"]),
                                            _ptr(out["ret_rank"]), _ptr(out["ret_row"]), _ptr(out["u_base"]), _stream())
     _lib.check(rc, "moe_ep_plan_dedup")
@@ -542,7 +555,7 @@ def ep_dispatch_dedup(x: torch.Tensor, perm: torch.Tensor, idx32: torch.Tensor, 
     """De-duplicated dispatch: every (token, destination rank) row once, plus the received-row number of every
     routed entry into the destination's index list (peer stores)."""
     _need_cuda(x, perm, urank, u_base)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = _lib.load().moe_ep_dispatch_dedup(_ptr(x), _ptr(perm), _ptr(idx32), _ptr(id_map), _ptr(offsets), _ptr(dst_base),
                                                _ptr(urank), _ptr(u_base), k, e_local, perm.numel(), x.shape[0], x.shape[1],
                                                peer_recv_ptrs, peer_gidx_ptrs, len(peer_recv_ptrs), _stream())
@@ -552,7 +565,7 @@ def ep_dispatch_dedup(x: torch.Tensor, perm: torch.Tensor, idx32: torch.Tensor, 
 def ep_barrier(peer_flag_ptrs, rank: int, channel: int, epoch: int, device: torch.device,
                timeout_us: int = 1_000_000) -> None:
     """Enqueue the time-limited barrier of the expert-parallel group on the current stream (see the header)."""
-    with torch.cuda.device(device):
+    with _on(device):
         rc = _lib.load().moe_ep_barrier(peer_flag_ptrs, len(peer_flag_ptrs), rank, channel, epoch, timeout_us,
                                         _ptr(status_buffer(device)), _stream())
     _lib.check(rc, "moe_ep_barrier")
@@ -567,7 +580,7 @@ def ep_share_counts(counts: torch.Tensor, extra: Optional[torch.Tensor], peer_ta
         raise ValueError("counts must be a contiguous int32 vector")
     if extra is not None and (extra.dtype != torch.int32 or not extra.is_contiguous() or extra.device != counts.device):
         raise ValueError("extra must be a contiguous int32 vector on the same device")
-    with torch.cuda.device(counts.device):
+    with _on(counts.device):
         rc = _lib.load().moe_ep_share_counts(_ptr(counts), counts.numel(), _ptr(extra), 0 if extra is None else extra.numel(),
                                              peer_table_ptrs, slot, peer_flag_ptrs, len(peer_flag_ptrs), rank, channel,
                                              epoch, timeout_us, _ptr(status_buffer(counts.device)), _stream())
@@ -579,7 +592,7 @@ def debug_bounds_status(device: torch.device):
     through MOE_B200_LIBRARY) recorded since the last call; the normal build reports (False, [0, 0, 0])."""
     import ctypes
     out = (ctypes.c_int32 * 3)()
-    with torch.cuda.device(device):
+    with _on(device):
         rc = _lib.load().moe_debug_bounds_status(out, _stream())
     if rc < 0:
         _lib.check(rc, "moe_debug_bounds_status")
@@ -589,7 +602,7 @@ def debug_bounds_status(device: torch.device):
 def debug_wait_probe(device: torch.device, limit_us: int = 1000) -> int:
     """Run the bounded-wait self-test kernel; returns 1 if the wait succeeded (it cannot), 0 if it ran out."""
     outcome = torch.full((1,), -1, dtype=torch.int32, device=device)
-    with torch.cuda.device(device):
+    with _on(device):
         rc = _lib.load().moe_debug_wait_probe(limit_us, _ptr(status_buffer(device)), _ptr(outcome), _stream())
     _lib.check(rc, "moe_debug_wait_probe")
     return int(outcome.item())
@@ -603,7 +616,7 @@ def grouped_gemm_peer_scatter(A: torch.Tensor, B: torch.Tensor, offsets: torch.T
     rows, K = A.shape
     E, N, _ = B.shape
     arr = peer_ptrs if not isinstance(peer_ptrs, (list, tuple)) else _ptr_array(peer_ptrs)
-    with torch.cuda.device(A.device):
+    with _on(A.device):
         rc = _lib.load().moe_grouped_gemm_peer_scatter(_ptr(A), _ptr(B), _ptr(offsets), _ptr(row_rank), _ptr(dst_rows),
                                                        arr, len(arr), ldy, rows if max_rows is None else max_rows,
                                                        expected_rows, K, N, E, _dtype_code(A, B),
