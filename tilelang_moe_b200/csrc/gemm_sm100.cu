@@ -431,6 +431,7 @@ __device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(
 // either) and adds up the softmax denominator; those, a dozen as a rule, go through the list in column order.  A warp
 // with more than ROUTER_CAP of them in one row feeds the list from tensor memory after all.
 constexpr int ROUTER_CAP = 16;
+static_assert((ROUTER_CAP + 1) * 256 <= 32 * Cfg<1, 128>::STAGING_PITCH, "parked logits of a warp fit its staging rows");
 __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t taddr, int grow, bool row_ok,
                                                     unsigned char* park, int lane) {
   constexpr int KMAX = 8;
@@ -474,7 +475,11 @@ __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t ta
   for (int j = 1; j < KMAX; ++j) V = j < p.r_k ? s[j] : V;
   const float top = s[0];
 
-  float2* mine = reinterpret_cast<float2*>(park) + lane;      // entry j of this row at mine[32 * j]
+  // Entry j of this row lies 256 * j bytes behind the row's first; entry ROUTER_CAP takes whatever does not fit.  Stores and
+  // counts are predicated: a branch per logit cost more than all the rest of this pass.
+  const uint32_t first = smem_u32(park) + lane * 8, last = first + ROUTER_CAP * 256;
+  const float2* mine = reinterpret_cast<const float2*>(park) + lane;
+  uint32_t at = first;
   int cnt = 0;
   double total = 0.0;                      // 32-term fp32 sums added up in fp64: the denominator of up to 256 terms
 #pragma unroll 1                            // keeps the scores within 1e-6 of an exactly summed softmax
@@ -482,21 +487,30 @@ __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t ta
     uint32_t v[32];
     tmem_ld32(taddr + c * 32, v);
     tmem_ld_wait();
+    float part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float x = __uint_as_float(v[j]);
-      if (!(x < V) && c * 32 + (j & ~7) < p.N) {
-        if (cnt < ROUTER_CAP) mine[32 * cnt] = make_float2(x, __int_as_float(c * 32 + j));
-        ++cnt;
+    for (int q = 0; q < 4; ++q) {
+      if (c * 32 + q * 8 < p.N) {           // N % 8 == 0
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          asm volatile(
+              "{\n\t.reg .pred p;\n\t"
+              "setp.geu.f32 p, %2, %3;\n\t"                 // not below V: also true for NaN
+              "@p st.shared.v2.b32 [%0], {%4, %5};\n\t"
+              "@p add.s32 %1, %1, 1;\n\t"
+              "@p add.u32 %0, %0, 256;\n\t"
+              "min.u32 %0, %0, %6;\n\t}"
+              : "+r"(at), "+r"(cnt)
+              : "f"(__uint_as_float(v[8 * q + j])), "f"(V), "r"(v[8 * q + j]), "r"(c * 32 + q * 8 + j), "r"(last)
+              : "memory");
+        }
+        if (p.r_mode != MOE_TOPK_MODE_B) {  // the conventions that normalise over all experts
+#pragma unroll
+          for (int j = 0; j < 8; ++j) part[q] += expf(__uint_as_float(v[8 * q + j]) - top);
+        }
       }
     }
-    if (p.r_mode != MOE_TOPK_MODE_B) {      // the conventions that normalise over all experts
-      float part = 0.f;
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (c * 32 + j < p.N) part += expf(__uint_as_float(v[j]) - top);
-      total += (double)part;
-    }
+    total += (double)((part[0] + part[1]) + (part[2] + part[3]));
   }
   int kv[KMAX], ki[KMAX];
 #pragma unroll
@@ -1479,7 +1493,8 @@ int moe::router_topk_gemm(const void* x, const void* Wr, int64_t T, int H, int E
     // instead of once per 128 (every CTA reads all of it, 48 KB per 64 columns of K with its own rows, 32 KB here), and
     // that traffic took as long as HBM's.
     // Measured (us; 16384 tokens, H = 7168, E = 256, k = 8, mode A): single CTAs, a list fed with every logit 97; pairs and
-    // parked logits 82 (HBM 36; the tensor pipe of the 128 SMs that hold a tile 44).
+    // parked logits 82, with predicated parking 69 (HBM 36; the tensor pipe of the 128 SMs that hold a tile 44).  What is
+    // left beside the tensor pipe is the epilogue of the one tile per CTA, which nothing overlaps.
     rc = make_tmap(&tB, Wr, (uint64_t)H, (uint64_t)E, 1, 128u, f16);
     if (rc) return rc;
     const int64_t units = (T + 2 * BM - 1) / (2 * BM);
