@@ -6,12 +6,12 @@
 //   * topk_lane_kernel   the same with one lane per row, staged through shared memory; N <= 32.
 //   * topk_warp_kernel   one warp per row, the row lives in registers; k rounds of
 //                        warp-wide arg-max by redux; N <= 1024, k <= 64.
-//   * topk_radix_kernel  a thread-block cluster per row; each CTA stages its slice
-//                        of the row in shared memory once, the cluster runs a
-//                        3-pass (11/11/10 bit) radix select on order-preserving
-//                        keys with histograms combined over distributed shared
-//                        memory, the selected entries are gathered into the leading
-//                        CTA, sorted (bitonic, 64-bit key|index) and normalised.
+//   * topk_radix_kernel  a thread-block cluster per row; each CTA keeps its share of
+//                        the row in registers, the cluster runs a radix select on
+//                        order-preserving keys with histograms combined over
+//                        distributed shared memory until few enough are left, every
+//                        CTA sorts its part (bitonic, 64-bit key|index) and places
+//                        it by binary search in the other CTAs' parts.
 // All read every logit once from HBM.
 //
 // Ordering contract: descending by value, equal values lowest index first,
@@ -569,7 +569,7 @@ constexpr int RWARPS = RT / 32;
 constexpr int RBINS = 2048;         // histogram bins (11-bit digit)
 constexpr int RBPT = RBINS / RT;    // bins owned by one thread in the scan (4)
 constexpr int RCTRL_BYTES = 256;
-constexpr int RMAX_SLICE = 16384;   // keys one CTA stages (64 KB)
+constexpr int RMAX_SLICE = 16384;   // keys one CTA holds (32 per thread)
 constexpr int RMAX_KPAD = 4096;
 
 struct RadixCtrl {
@@ -577,11 +577,11 @@ struct RadixCtrl {
   double warp_d[RWARPS];
   uint32_t sel_bin;
   uint32_t k_rem;
-  uint32_t sel_count;
+  uint32_t bin_count;   // entries of the selected bin in the whole row
   uint32_t blk_maxkey;
-  uint32_t loc_count;   // selected entries compacted in this CTA
-  uint32_t loc_base;    // their first slot in the leading CTA's buffer
-  double blk_sum;
+  uint32_t loc_count;   // collected entries of this CTA
+  double blk_sum;       // this CTA's share of the full-row denominator (modes A)
+  double sel_sum;       // ... of a sum over the k selected
 };
 static_assert(sizeof(RadixCtrl) <= RCTRL_BYTES, "control block too large");
 
@@ -664,9 +664,33 @@ __device__ __forceinline__ void block_sort_desc(uint64_t* sbuf, int tid) {
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(RT)
-topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld, int k, int kpad, int mode,
-                  int slice, int vec_ok, float* __restrict__ scores, int64_t* __restrict__ idx64,
+// entries of the descending list a[0 .. n) that are greater than x
+__device__ __forceinline__ uint32_t count_above(const uint64_t* a, uint32_t n, uint64_t x) {
+  uint32_t lo = 0u, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (a[mid] > x) lo = mid + 1u; else hi = mid;
+  }
+  return lo;
+}
+
+// One cluster of C CTAs per row.  The row's 128-byte chunks go round the CTAs (a row in sorted order is spread evenly), each
+// keeps its share as keys in registers, KPT per thread.
+//   1. radix select on key | column, 11 / 11 / 10 bits of the key, then 11 / 6 of the column among equal keys: histograms of
+//      all CTAs are added over distributed shared memory.  It stops as soon as the entries not below the selected bin are
+//      few enough to be sorted outright (totcap), after one digit as a rule.
+//   2. every CTA collects those of its share and sorts them;
+//   3. it copies the other CTAs' sorted entries; an entry's place in the row's order is its place in its own list plus, by
+//      binary search, the entries of the other lists ahead of it.  Places below k are written out.
+// What bounds it: latency (barriers, shared-memory atomics, the sort's chain of exchanges).
+// Measured (us, gathering the k selected into the leading CTA and sorting them there after all three digits -> this):
+// 64 x 32768, k = 2048: 44.0 -> 31.4; one such row 30.4 -> 19.6; 4096 x 4096, k = 64: 177 -> 140; 256 x 32768, k = 2048:
+// 100 -> 93; 16 x 65536, k = 1024: 34.9 -> 26.1; 64 x 32768, k = 32: 19.8 -> 16.8.  Rows of equal logits alone pay for the
+// two more digits: 64 x 32768, k = 32 20.2 -> 27.1, k = 2048 45.5 -> 33.5.
+template <int KPT>
+__global__ void __launch_bounds__(RT, 2)
+topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld, int k, int totcap, int lcap, int mode,
+                  int vec_ok, float* __restrict__ scores, int64_t* __restrict__ idx64,
                   int32_t* __restrict__ idx32, int32_t* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_trigger();
@@ -678,61 +702,69 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
 
   RadixCtrl* ctrl = reinterpret_cast<RadixCtrl*>(smem_raw);
   uint32_t* hist = reinterpret_cast<uint32_t*>(smem_raw + RCTRL_BYTES);
-  uint64_t* sbuf = reinterpret_cast<uint64_t*>(smem_raw + RCTRL_BYTES + 2 * RBINS * 4);
-  uint64_t* lbuf = sbuf + kpad;                      // this CTA's selected entries before they go to the leader
-  uint32_t* keys = reinterpret_cast<uint32_t*>(lbuf + kpad);
+  uint64_t* lbuf = reinterpret_cast<uint64_t*>(smem_raw + RCTRL_BYTES + 2 * RBINS * 4);   // [lcap] this CTA's entries
+  uint64_t* others = lbuf + lcap;                                                         // [totcap] the other CTAs'
 
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  const int begin = (int)crank * slice;
-  int len = N - begin;
-  if (len > slice) len = slice;
-  if (len < 0) len = 0;
-
-  if (tid == 0) { ctrl->sel_count = 0u; ctrl->blk_maxkey = 0u; ctrl->blk_sum = 0.0; ctrl->sel_bin = 0u; ctrl->k_rem = 0u; }
+  if (tid == 0) { ctrl->blk_maxkey = 0u; ctrl->blk_sum = 0.0; ctrl->sel_bin = 0u; ctrl->k_rem = 0u; ctrl->bin_count = 0u; }
   for (int i = tid; i < 2 * RBINS; i += RT) hist[i] = 0u;
-  if (crank == 0)
-    for (int i = k + tid; i < kpad; i += RT) sbuf[i] = 0ull;
 
-  // ---- stage the slice as keys (the only read of the logits)
-  const float* p = logits + row * ld + begin;
-  uint32_t lmax = 0u;
-  if (vec_ok) {
-    for (int i = tid * 4; i < len; i += RT * 4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(p + i));
-      uint4 kk;
-      kk.x = float_to_key(v.x); kk.y = float_to_key(v.y); kk.z = float_to_key(v.z); kk.w = float_to_key(v.w);
-      *reinterpret_cast<uint4*>(keys + i) = kk;
-      lmax = max(max(lmax, kk.x), max(kk.y, max(kk.z, kk.w)));
-    }
-  } else {
-    for (int i = tid; i < len; i += RT) {
-      const uint32_t kk = float_to_key(__ldg(p + i));
-      keys[i] = kk;
-      lmax = max(lmax, kk);
+  // ---- this CTA's share as keys (the only read of the logits); 0 where there is none (no float has that key)
+  const float* p = logits + row * ld;
+  auto col_of = [&](int j) {                          // column of key j of this thread
+    const int v = (j >> 2) * RT + tid;                // vector of four in the CTA's share, eight to a chunk
+    return (((v >> 3) * (int)C + (int)crank) << 5) + ((v & 7) << 2) + (j & 3);
+  };
+  uint32_t key[KPT];
+#pragma unroll
+  for (int q = 0; q < KPT / 4; ++q) {
+    const int i = col_of(4 * q);
+    if (vec_ok) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      const bool in = i < N;                          // N % 4 == 0 on this path
+      if (in) v = __ldg(reinterpret_cast<const float4*>(p + i));
+      key[4 * q] = in ? float_to_key(v.x) : 0u;
+      key[4 * q + 1] = in ? float_to_key(v.y) : 0u;
+      key[4 * q + 2] = in ? float_to_key(v.z) : 0u;
+      key[4 * q + 3] = in ? float_to_key(v.w) : 0u;
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) key[4 * q + c] = i + c < N ? float_to_key(__ldg(p + i + c)) : 0u;
     }
   }
-  __syncthreads();  // ctrl initialised, keys staged
+  __syncthreads();  // control block and histograms initialised
   if (mode != MOE_TOPK_MODE_B) {
+    uint32_t lmax = 0u;
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) lmax = max(lmax, key[j]);
     lmax = __reduce_max_sync(FULL, lmax);
     if (lane == 0) atomicMax(&ctrl->blk_maxkey, lmax);
   }
 
-  // ---- radix select: after three passes `prefix` is the key of the k-th largest value
-  uint32_t prefix = 0u, pmask = 0u, k_rem = (uint32_t)k, bin = 0u;
+  // ---- 1. radix select: `prefix` is the lowest key of the bin that holds the k-th largest entry (after three digits its key),
+  //      `cprefix` the same of CMAX - column among equal keys
+  constexpr int CMAX = (1 << 17) - 1;                 // N <= 8 * RMAX_SLICE = 2^17
+  uint32_t prefix = 0u, pmask = 0u, cprefix = 0u, cmask = 0u, k_rem = (uint32_t)k;
   double rowsum = 0.0;
-  uint32_t* h = hist;
-  for (int pass = 0; pass < 3; ++pass) {
-    const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
-    const uint32_t dmask = pass == 2 ? 1023u : 2047u;
-    h = hist + (pass & 1) * RBINS;
-    if (pass == 2) {  // buffer 0 again: every remote read of pass 0 ended before pass 1's cluster barrier
+#pragma unroll 1
+  for (int pass = 0; pass < 5; ++pass) {
+    const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : (pass == 3 ? 6 : 0));
+    const uint32_t dmask = pass == 2 ? 1023u : (pass == 4 ? 63u : 2047u);
+    uint32_t* h = hist + (pass & 1) * RBINS;
+    if (pass >= 2) {  // this buffer again: every remote read of it ended before the last pass's cluster barrier
       for (int i = tid; i < RBINS; i += RT) h[i] = 0u;
       __syncthreads();
     }
-    for (int i = tid; i < len; i += RT) {
-      const uint32_t kk = keys[i];
-      if ((kk & pmask) == prefix) atomicAdd(&h[(kk >> shift) & dmask], 1u);
+    if (pass < 3) {
+#pragma unroll
+      for (int j = 0; j < KPT; ++j)
+        if (key[j] != 0u && (key[j] & pmask) == prefix) atomicAdd(&h[(key[j] >> shift) & dmask], 1u);
+    } else {
+#pragma unroll
+      for (int j = 0; j < KPT; ++j) {
+        const uint32_t inv = (uint32_t)(CMAX - col_of(j));
+        if (key[j] == prefix && (inv & cmask) == cprefix) atomicAdd(&h[(inv >> shift) & dmask], 1u);
+      }
     }
     cluster.sync();
 
@@ -760,14 +792,19 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
     for (int w = wid + 1; w < RWARPS; ++w) S += ctrl->warp_tot[w];
 #pragma unroll
     for (int j = RBPT - 1; j >= 0; --j) {
-      if (S < k_rem && k_rem <= S + g[j]) { ctrl->sel_bin = (uint32_t)(tid * RBPT + j); ctrl->k_rem = k_rem - S; }
+      if (S < k_rem && k_rem <= S + g[j]) {
+        ctrl->sel_bin = (uint32_t)(tid * RBPT + j);
+        ctrl->k_rem = k_rem - S;
+        ctrl->bin_count = g[j];
+      }
       S += g[j];
     }
     __syncthreads();
-    bin = ctrl->sel_bin;
+    const uint32_t bin = ctrl->sel_bin;
     k_rem = ctrl->k_rem;
-    prefix |= bin << shift;
-    pmask |= dmask << shift;
+    const uint32_t total_ge = (uint32_t)k - k_rem + ctrl->bin_count;
+    if (pass < 3) { prefix |= bin << shift; pmask |= dmask << shift; }
+    else { cprefix |= bin << shift; cmask |= dmask << shift; }
 
     if (pass == 0 && mode != MOE_TOPK_MODE_B) {
       // full-row softmax denominator: cluster max, then this CTA's share of sum exp(v - max)
@@ -775,128 +812,160 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
       for (unsigned c = 0; c < C; ++c) gmax = max(gmax, cluster.map_shared_rank(ctrl, c)->blk_maxkey);
       const float vmax = key_to_float(gmax);
       double part = 0.0;
-      for (int i = tid; i < len; i += RT) part += (double)expf(key_to_float(keys[i]) - vmax);
+#pragma unroll
+      for (int j = 0; j < KPT; ++j)
+        if (key[j] != 0u) part += (double)expf(key_to_float(key[j]) - vmax);
       part = block_sum_ordered(part, ctrl, lane, wid);
       if (tid == 0) ctrl->blk_sum = part;  // published by the next cluster barrier
     }
-  }
-  const uint32_t thr = prefix;        // key of the k-th largest element
-  const uint32_t need_eq = k_rem;     // how many entries equal to it are taken (lowest indices first)
-
-  // equal-to-threshold entries per CTA sit in the last histogram; CTAs hold ascending index ranges
-  uint32_t eq_before = 0u;
-  const uint32_t eq_local = h[bin];
-  for (unsigned c = 0; c < crank; ++c) eq_before += cluster.map_shared_rank(h, c)[bin];
-  uint32_t take = 0u;
-  if (need_eq > eq_before) { take = need_eq - eq_before; if (take > eq_local) take = eq_local; }
-  const bool take_all = (take == eq_local);
-  if (mode != MOE_TOPK_MODE_B && crank == 0) {
-    for (unsigned c = 0; c < C; ++c) rowsum += cluster.map_shared_rank(ctrl, c)->blk_sum;
+    if (total_ge <= (uint32_t)totcap) break;          // the same in every CTA of the cluster; all five digits leave k entries
+    __syncthreads();                                  // every thread has read the selection before the next pass replaces it
   }
 
-  // ---- gather the selected entries into the leading CTA: compact them locally first (shared-memory atomics are
-  //      cheap, remote ones are not), reserve their place in the leader's buffer with one remote atomic, copy
-  uint64_t* lead_sbuf = cluster.map_shared_rank(sbuf, 0);
-  uint32_t* lead_count = cluster.map_shared_rank(&ctrl->sel_count, 0);
-  if (tid == 0) ctrl->loc_count = 0u;
-  __syncthreads();
-  for (int base = 0; base < len; base += RT) {
-    const int i = base + tid;
-    const uint32_t kk = i < len ? keys[i] : 0u;
-    const bool sel = i < len && (kk > thr || (take_all && kk == thr));
-    const unsigned m = __ballot_sync(FULL, sel);
-    if (m) {
-      uint32_t b = 0u;
-      if (lane == 0) b = atomicAdd(&ctrl->loc_count, (uint32_t)__popc(m));
-      b = __shfl_sync(FULL, b, 0);
-      if (sel) lbuf[b + __popc(m & lt_mask)] = pack_entry(kk, (uint32_t)(begin + i));
-    }
+  // ---- 2. collect
+  uint32_t m = 0u;
+#pragma unroll
+  for (int j = 0; j < KPT; ++j) {
+    const bool in = key[j] > prefix || (key[j] == prefix && (uint32_t)(CMAX - col_of(j)) >= cprefix);
+    m |= (key[j] != 0u && in) ? (1u << j) : 0u;
   }
-  if (!take_all && take > 0u) {  // block-uniform: only the first `take` equal entries, in index order
-    uint32_t running = 0u;
-    for (int base = 0; base < len && running < take; base += RT) {
-      const int i = base + tid;
-      const bool eq = i < len && keys[i] == thr;
-      const unsigned m = __ballot_sync(FULL, eq);
-      __syncthreads();
-      if (lane == 0) ctrl->warp_tot[wid] = (uint32_t)__popc(m);
-      __syncthreads();
-      uint32_t before = running, total = 0u;
-      for (int w = 0; w < RWARPS; ++w) {
-        const uint32_t t = ctrl->warp_tot[w];
-        if (w < wid) before += t;
-        total += t;
-      }
-      const uint32_t myrank = before + (uint32_t)__popc(m & lt_mask);
-      if (eq && myrank < take) {
-        const uint32_t slot = atomicAdd(&ctrl->loc_count, 1u);
-        lbuf[slot] = pack_entry(thr, (uint32_t)(begin + i));
-      }
-      running += total;
-    }
-  }
-  __syncthreads();
-  if (tid == 0) ctrl->loc_base = atomicAdd(lead_count, ctrl->loc_count);
-  __syncthreads();
+  uint32_t total = 0u;
   {
-    const uint32_t cnt = ctrl->loc_count, base0 = ctrl->loc_base;
-    for (uint32_t i = tid; i < cnt; i += RT) lead_sbuf[base0 + i] = lbuf[i];
+    const uint32_t n = (uint32_t)__popc(m);
+    uint32_t inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, inc, o);
+      if (lane >= o) inc += v;
+    }
+    __syncthreads();
+    if (lane == 31) ctrl->warp_tot[wid] = inc;
+    __syncthreads();
+    uint32_t slot = inc - n;
+#pragma unroll
+    for (int w = 0; w < RWARPS; ++w) {
+      const uint32_t t = ctrl->warp_tot[w];
+      if (w < wid) slot += t;
+      total += t;
+    }
+#pragma unroll
+    for (int j = 0; j < KPT; ++j)
+      if ((m >> j) & 1u) lbuf[slot++] = pack_entry(key[j], (uint32_t)col_of(j));
   }
-  cluster.sync();
-  if (crank != 0) return;  // nobody reads another CTA's shared memory past this point
-
-  if (tid == 0 && ctrl->sel_count != (uint32_t)k && status) {
-    status[0] = ST_INTERNAL; status[1] = (int32_t)ctrl->sel_count; status[2] = (int32_t)row;
-  }
-
-  // ---- bitonic sort, descending, of kpad 64-bit entries (padding entries are 0 and sink to the end):
-  //      in registers + shuffles when there is at least one entry per thread, else the plain shared-memory network
-  if (kpad >= RT) {   // block-uniform
-    if (kpad == RT) block_sort_desc<1>(sbuf, tid);
-    else if (kpad == 2 * RT) block_sort_desc<2>(sbuf, tid);
-    else if (kpad == 4 * RT) block_sort_desc<4>(sbuf, tid);
-    else block_sort_desc<8>(sbuf, tid);
+  // ---- sort, descending; unused places are 0 and sink to the end.  From 129 entries on in registers and shuffles,
+  //      below that the plain shared-memory network
+  int size = 2;
+  while (size < (int)total) size <<= 1;
+  if (size > 128 && size < RT) size = RT;
+  for (int i = (int)total + tid; i < size; i += RT) lbuf[i] = 0ull;
+  if (tid == 0) ctrl->loc_count = total;
+  __syncthreads();
+  if (size >= RT) {   // block-uniform
+    if (size == RT) block_sort_desc<1>(lbuf, tid);
+    else if (size == 2 * RT) block_sort_desc<2>(lbuf, tid);
+    else if (size == 4 * RT) block_sort_desc<4>(lbuf, tid);
+    else block_sort_desc<8>(lbuf, tid);
   } else {
-    for (int size = 2; size <= kpad; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int t = tid; t < (kpad >> 1); t += RT) {
+    for (int sz = 2; sz <= size; sz <<= 1) {
+      for (int stride = sz >> 1; stride > 0; stride >>= 1) {
+        for (int t = tid; t < (size >> 1); t += RT) {
           const int i = 2 * t - (t & (stride - 1));
           const int j = i + stride;
-          const bool desc = (i & size) == 0;
-          const uint64_t a = sbuf[i], b = sbuf[j];
-          if ((a < b) == desc) { sbuf[i] = b; sbuf[j] = a; }
+          const bool desc = (i & sz) == 0;
+          const uint64_t a = lbuf[i], b = lbuf[j];
+          if ((a < b) == desc) { lbuf[i] = b; lbuf[j] = a; }
         }
         __syncthreads();
       }
     }
   }
 
-  // ---- softmax over the k selected (mode B) or against the full-row denominator (modes A)
-  const float vmax = key_to_float((uint32_t)(sbuf[0] >> 32));
-  float denom;
-  if (mode == MOE_TOPK_MODE_B) {
-    double part = 0.0;
-    for (int r = tid; r < k; r += RT) part += (double)expf(key_to_float((uint32_t)(sbuf[r] >> 32)) - vmax);
-    denom = (float)block_sum_ordered(part, ctrl, lane, wid);
-  } else {
-    denom = (float)rowsum;
+  // ---- 3. the other CTAs' entries, and every entry's place in the row
+  uint32_t cnt[8], all = total;
+  float vmax = key_to_float((uint32_t)(lbuf[0] >> 32));
+  rowsum = ctrl->blk_sum;
+  if (C > 1) {
+    cluster.sync();                                   // sorted lists, counts and denominators of all CTAs are there
+    uint32_t at = 0u, top = 0u;
+    all = 0u;
+    rowsum = 0.0;
+#pragma unroll
+    for (unsigned c = 0; c < 8; ++c) {
+      cnt[c] = 0u;
+      if (c < C) {
+        const RadixCtrl* rc = cluster.map_shared_rank(ctrl, c);
+        const uint32_t n = rc->loc_count;
+        rowsum += rc->blk_sum;
+        const uint64_t* rl = cluster.map_shared_rank(lbuf, c);
+        if (n > 0u) top = max(top, (uint32_t)(rl[0] >> 32));
+        all += n;
+        if (c != crank) {
+          for (uint32_t i = tid; i < n; i += RT) others[at + i] = rl[i];
+          cnt[c] = n;
+          at += n;
+        }
+      }
+    }
+    vmax = key_to_float(top);
+    __syncthreads();
+  }
+  if (tid == 0 && crank == 0 && all < (uint32_t)k && status) {
+    status[0] = ST_INTERNAL; status[1] = (int32_t)all; status[2] = (int32_t)row;
+  }
+  auto place = [&](uint32_t i, uint64_t ent) {        // entry i of this CTA's list
+    uint32_t r = i, at = 0u;
+    if (C > 1) {
+#pragma unroll
+      for (unsigned c = 0; c < 8; ++c)
+        if (c < C) { r += count_above(others + at, cnt[c], ent); at += cnt[c]; }
+    }
+    return r;
+  };
+  constexpr int EMAX = 8;                             // RMAX_KPAD / RT entries per thread at most
+  uint32_t rank[EMAX];
+  double part = 0.0;
+#pragma unroll
+  for (int e = 0; e < EMAX; ++e) {
+    const uint32_t i = (uint32_t)(e * RT + tid);
+    rank[e] = 0xFFFFFFFFu;
+    if (i < total) {
+      const uint64_t ent = lbuf[i];
+      rank[e] = place(i, ent);
+      if (mode == MOE_TOPK_MODE_B && rank[e] < (uint32_t)k) part += (double)expf(key_to_float((uint32_t)(ent >> 32)) - vmax);
+    }
+  }
+  float denom = (float)rowsum;
+  if (mode == MOE_TOPK_MODE_A_RENORM) {
+#pragma unroll
+    for (int e = 0; e < EMAX; ++e)
+      if (rank[e] < (uint32_t)k)
+        part += (double)(expf(key_to_float((uint32_t)(lbuf[e * RT + tid] >> 32)) - vmax) / denom);
   }
   float renorm = 1.f;
-  if (mode == MOE_TOPK_MODE_A_RENORM) {
-    double part = 0.0;
-    for (int r = tid; r < k; r += RT) part += (double)(expf(key_to_float((uint32_t)(sbuf[r] >> 32)) - vmax) / denom);
-    renorm = (float)block_sum_ordered(part, ctrl, lane, wid);
+  if (mode != MOE_TOPK_MODE_A) {                      // a sum over the k selected, added up over the cluster
+    double sum = block_sum_ordered(part, ctrl, lane, wid);
+    if (C > 1) {
+      if (tid == 0) ctrl->sel_sum = sum;
+      cluster.sync();
+      sum = 0.0;
+      for (unsigned c = 0; c < C; ++c) sum += cluster.map_shared_rank(ctrl, c)->sel_sum;
+    }
+    if (mode == MOE_TOPK_MODE_B) denom = (float)sum; else renorm = (float)sum;
   }
   const int64_t o = row * (int64_t)k;
-  for (int r = tid; r < k; r += RT) {
-    const uint64_t ent = sbuf[r];
-    float s = expf(key_to_float((uint32_t)(ent >> 32)) - vmax) / denom;
-    if (mode == MOE_TOPK_MODE_A_RENORM) s = s / renorm;
-    const uint32_t col = 0xFFFFFFFFu - (uint32_t)(ent & 0xFFFFFFFFull);
-    scores[o + r] = s;
-    if (idx64) idx64[o + r] = (int64_t)col;
-    if (idx32) idx32[o + r] = (int32_t)col;
+#pragma unroll
+  for (int e = 0; e < EMAX; ++e) {
+    if (rank[e] < (uint32_t)k) {
+      const uint64_t ent = lbuf[e * RT + tid];
+      float s = expf(key_to_float((uint32_t)(ent >> 32)) - vmax) / denom;
+      if (mode == MOE_TOPK_MODE_A_RENORM) s = s / renorm;
+      const uint32_t col = 0xFFFFFFFFu - (uint32_t)(ent & 0xFFFFFFFFull);
+      scores[o + rank[e]] = s;
+      if (idx64) idx64[o + rank[e]] = (int64_t)col;
+      if (idx32) idx32[o + rank[e]] = (int32_t)col;
+    }
   }
+  if (C > 1) cluster.sync();                          // nobody leaves while its shared memory is still read
 }
 
 static int next_pow2(int v) {
@@ -907,18 +976,28 @@ static int next_pow2(int v) {
 
 static int launch_radix(const float* logits, int64_t M, int N, int64_t ld, int k, int mode, float* scores,
                         int64_t* idx64, int32_t* idx32, int32_t* status, const DeviceInfo& dev, cudaStream_t st) {
-  // cluster size: a slice must fit; beyond that split rows until the grid covers the SMs
+  // cluster size: a share must fit 32 keys per thread; beyond that split rows until the grid covers the SMs
+  const int chunks = (N + 31) / 32;
   int C = 1;
-  while (C < 8 && ((N + C - 1) / C > RMAX_SLICE || (M * C < dev.sm_count && N / (2 * C) >= 2048))) C <<= 1;
-  int slice = (N + C - 1) / C;
-  slice = (slice + 3) & ~3;
+  while (C < 8 && ((chunks + C - 1) / C * 32 > RMAX_SLICE || (M * C < dev.sm_count && N / (2 * C) >= 2048))) C <<= 1;
+  const int slice = (chunks + C - 1) / C * 32;
   if (slice > RMAX_SLICE) return fail(MOE_ERR_UNSUPPORTED, "topk_softmax: N=%d exceeds %d", N, 8 * RMAX_SLICE);
   int kpad = next_pow2(k);
   if (kpad < 2) kpad = 2;
   if (kpad > RMAX_KPAD) return fail(MOE_ERR_UNSUPPORTED, "topk_softmax: k=%d exceeds %d", k, RMAX_KPAD);
-  const size_t smem = (size_t)RCTRL_BYTES + 2 * RBINS * 4 + (size_t)kpad * 16 + (size_t)slice * 4;
+  // Entries a row may hand to the sort.  One CTA: what a sort of k entries (or of RT) takes anyway.  More CTAs: three
+  // quarters of the length their shares of k, with a quarter on top, round up to.
+  int totcap = kpad > RT ? kpad : RT;
+  if (C > 1) {
+    const int share = 3 * C * next_pow2((k + k / 4) / C + 1) / 4;
+    if (share > totcap) totcap = share;
+    if (totcap > RMAX_KPAD) totcap = RMAX_KPAD;
+  }
+  const int lcap = next_pow2(totcap);
+  const size_t smem = (size_t)RCTRL_BYTES + 2 * RBINS * 4 + (size_t)lcap * 8 + (C > 1 ? (size_t)totcap * 8 : 0);
   const int vec_ok = (N % 4 == 0) && (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
-  MOE_CUDA_CHECK(cudaFuncSetAttribute(topk_radix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto kernel = slice <= 8 * RT ? topk_radix_kernel<8> : (slice <= 16 * RT ? topk_radix_kernel<16> : topk_radix_kernel<32>);
+  MOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(M * C), 1, 1);
@@ -932,7 +1011,7 @@ static int launch_radix(const float* logits, int64_t M, int N, int64_t ld, int k
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  MOE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, topk_radix_kernel, logits, M, N, ld, k, kpad, mode, slice, vec_ok, scores,
+  MOE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, logits, M, N, ld, k, totcap, lcap, mode, vec_ok, scores,
                                     idx64, idx32, status));
   return MOE_OK;
 }
