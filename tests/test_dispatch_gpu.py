@@ -70,3 +70,22 @@ def test_router_selection_in_the_epilogue(cuda, lib, T, E, k, kind):
         s_ref, i_ref = O.topk_softmax(lg.cpu(), k, mode)
         assert torch.equal(i.cpu(), i_ref)
         torch.testing.assert_close(s.cpu(), s_ref, rtol=1e-6, atol=1e-30)
+
+
+@pytest.mark.parametrize("T,H,E,k", [(1, 8, 1, 1), (3, 2048, 8, 2), (148, 264, 3, 3), (296, 2056, 16, 8), (297, 2048, 13, 4),
+                                     (20, 3000, 32, 32), (5, 4096, 24, 6), (64, 16, 9, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_few_experts_a_cta_or_a_warp_per_token(cuda, lib, T, H, E, k, dtype):
+    """CUDA-core router on both sides of its rule (a CTA per token up to two per SM): inputs on a coarse grid make every
+    product and sum exact in fp32, so both forms give the exact logits."""
+    g = torch.Generator().manual_seed(T + H + E)
+    X = (torch.round(torch.randn(T, H, generator=g) * 2) / 2).to(dtype)
+    W = (torch.round(torch.randn(E, H, generator=g) * 2) / 8).to(dtype)
+    lg = torch.full((T, E), float("nan"), device=cuda)
+    for mode in ("B", "A", "A_renorm"):
+        s, i = ops.router_topk_softmax(X.to(cuda), W.to(cuda), k, mode=mode, logits_out=lg, fused=True)
+        ops.check_status(cuda)
+        assert torch.equal(lg.cpu().double(), X.double() @ W.double().T)
+        s_ref, i_ref = O.topk_softmax(lg.cpu(), k, mode)
+        assert torch.equal(i.cpu(), i_ref)
+        torch.testing.assert_close(s.cpu(), s_ref, rtol=1e-6, atol=1e-30)

@@ -381,6 +381,35 @@ combine_kernel(const uint4* __restrict__ Yk, const uint4* __restrict__ shared, c
 // router logits for a small expert count: the router weight [E,H] is staged once per CTA in shared memory,
 // then each warp takes tokens in turn: one pass over the token row, all E dot products in registers
 // ------------------------------------------------------------------------------------
+// One warp, logit of expert `lane` in `mine` (E <= 32): stores it where asked to, then top-k + softmax for token t.
+__device__ __forceinline__ void router_select(float mine, int lane, int E, int k, int mode, int64_t t, float* logits,
+                                              float* scores, int64_t* idx64, int32_t* idx32) {
+  if (logits && lane < E) logits[t * E + lane] = mine;
+  if (k > 0) {
+    // fused top-k + softmax over the E <= 32 logits held one per lane: k rounds of warp arg-max, lowest
+    // lane first among equals; lane r keeps the r-th winner
+    const unsigned FULL = 0xFFFFFFFFu;
+    int key = lane < E ? float_to_ikey(mine) : (int)0x80000000;
+    int win_key = (int)0x80000000, win_idx = 0;
+    for (int r = 0; r < k; ++r) {
+      const int m = __reduce_max_sync(FULL, key);
+      const int sel = __ffs(__ballot_sync(FULL, key == m)) - 1;
+      if (lane == r) { win_key = m; win_idx = sel; }
+      if (lane == sel) key = (int)0x80000000;
+    }
+    const float vmax = ikey_to_float(__shfl_sync(FULL, win_key, 0));
+    const float e = lane < k ? expf(ikey_to_float(win_key) - vmax) : 0.f;
+    const float denom = mode == MOE_TOPK_MODE_B ? warp_sum(e) : warp_sum(lane < E ? expf(mine - vmax) : 0.f);
+    float sc = e / denom;
+    if (mode == MOE_TOPK_MODE_A_RENORM) sc = sc / warp_sum(sc);
+    if (lane < k) {
+      scores[t * k + lane] = sc;
+      if (idx64) idx64[t * k + lane] = (int64_t)win_idx;
+      if (idx32) idx32[t * k + lane] = (int32_t)win_idx;
+    }
+  }
+}
+
 template <bool F16, int EMAX>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const uint4* __restrict__ x, const uint4* __restrict__ Wr, int64_t T, int vec_per_row, int E,
@@ -440,30 +469,77 @@ router_logits_kernel(const uint4* __restrict__ x, const uint4* __restrict__ Wr, 
       const float sum = warp_sum(acc[j]);
       if (lane == j) mine = sum;
     }
-    if (logits && lane < E) logits[t * E + lane] = mine;
-    if (k > 0) {
-      // fused top-k + softmax over the E <= 32 logits held one per lane: k rounds of warp arg-max, lowest
-      // lane first among equals; lane r keeps the r-th winner
-      const unsigned FULL = 0xFFFFFFFFu;
-      int key = lane < E ? float_to_ikey(mine) : (int)0x80000000;
-      int win_key = (int)0x80000000, win_idx = 0;
-      for (int r = 0; r < k; ++r) {
-        const int m = __reduce_max_sync(FULL, key);
-        const int sel = __ffs(__ballot_sync(FULL, key == m)) - 1;
-        if (lane == r) { win_key = m; win_idx = sel; }
-        if (lane == sel) key = (int)0x80000000;
-      }
-      const float vmax = ikey_to_float(__shfl_sync(FULL, win_key, 0));
-      const float e = lane < k ? expf(ikey_to_float(win_key) - vmax) : 0.f;
-      const float denom = mode == MOE_TOPK_MODE_B ? warp_sum(e) : warp_sum(lane < E ? expf(mine - vmax) : 0.f);
-      float sc = e / denom;
-      if (mode == MOE_TOPK_MODE_A_RENORM) sc = sc / warp_sum(sc);
-      if (lane < k) {
-        scores[t * k + lane] = sc;
-        if (idx64) idx64[t * k + lane] = (int64_t)win_idx;
-        if (idx32) idx32[t * k + lane] = (int32_t)win_idx;
+    router_select(mine, lane, E, k, mode, t, logits, scores, idx64, idx32);
+  }
+}
+
+// The same logits for few tokens: one CTA per token, the row spread over its 256 threads, the router weight read from L2.
+// With a warp per token the staging of the weight and then the row, eight vectors per lane, stand in one chain.
+// The EMAX sums of a warp are reduced together: each exchange halves the number of sums a lane still carries.
+template <bool F16, int EMAX>
+__global__ void __launch_bounds__(256)
+router_token_kernel(const uint4* __restrict__ x, const uint4* __restrict__ Wr, int vec_per_row, int E,
+                    float* __restrict__ logits, int k, int mode, float* __restrict__ scores,
+                    int64_t* __restrict__ idx64, int32_t* __restrict__ idx32) {
+  __shared__ float part[8][32];
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t t = blockIdx.x;
+  const uint4* xr = x + t * vec_per_row;
+  float acc[EMAX];
+#pragma unroll
+  for (int j = 0; j < EMAX; ++j) acc[j] = 0.f;
+  for (int v = threadIdx.x; v < vec_per_row; v += 256) {
+    const uint4 xv = __ldg(xr + v);
+    uint4 wv[8];
+#pragma unroll
+    for (int j0 = 0; j0 < EMAX; j0 += 8) {            // eight experts' vectors in flight at a time
+#pragma unroll
+      for (int j = 0; j < 8; ++j) wv[j] = j0 + j < E ? __ldg(Wr + (int64_t)(j0 + j) * vec_per_row + v) : make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t* xu = reinterpret_cast<const uint32_t*>(&xv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t* wu = reinterpret_cast<const uint32_t*>(&wv[j]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 a = unpack2<F16>(xu[q]), b = unpack2<F16>(wu[q]);
+          acc[j0 + j] = fmaf(a.x, b.x, acc[j0 + j]);
+          acc[j0 + j] = fmaf(a.y, b.y, acc[j0 + j]);
+        }
       }
     }
+  }
+  // lanes whose bit d is set keep the upper half of the sums, the others the lower half: after log2(EMAX) exchanges lane l
+  // holds sum number bitrev(l) of its group, and the remaining exchanges add up the groups
+  int width = EMAX;
+#pragma unroll
+  for (int d = 1; d < EMAX; d <<= 1) {
+    width >>= 1;
+#pragma unroll
+    for (int j = 0; j < EMAX / 2; ++j) {
+      if (j < width) {
+        const bool up = (lane & d) != 0;
+        const float give = up ? acc[j] : acc[j + width], keep = up ? acc[j + width] : acc[j];
+        acc[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, d);
+      }
+    }
+  }
+  float sum = acc[0];
+#pragma unroll
+  for (int d = EMAX; d < 32; d <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
+  int e = 0;                                          // the expert whose sum this lane ended up with
+#pragma unroll
+  for (int d = 1, w = EMAX / 2; d < EMAX; d <<= 1, w >>= 1) e += (lane & d) ? w : 0;
+  if (lane < EMAX) part[warp][e] = sum;
+  __syncthreads();
+  if (warp == 0) {
+    float mine = 0.f;
+    if (lane < E) {
+#pragma unroll
+      for (int w = 0; w < 8; ++w) mine += part[w][lane];
+    }
+    router_select(mine, lane, E, k, mode, t, logits, scores, idx64, idx32);
   }
 }
 
@@ -672,11 +748,23 @@ static int router_small(const void* x, const void* Wr, int64_t T, int H, int E, 
   DeviceInfo dev;
   int rc = current_device_info(&dev);
   if (rc) return rc;
-  // one CTA per SM at most: every CTA stages the whole router weight
   const size_t smem = (size_t)E * H * 2;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  // Measured (us, H = 2048, E = 8): 8 tokens 6.8 with a warp per token, 3.4 with a CTA; 1024 tokens 7.2 either way, and the
+  // weight is read from L2 for every token: a CTA per token up to two per SM
+  if (T <= (int64_t)dev.sm_count * 2) {
+#define MOE_RT_LAUNCH(F16_, EMAX_)                                                                                       \
+    router_token_kernel<F16_, EMAX_><<<(unsigned)T, 256, 0, st>>>(reinterpret_cast<const uint4*>(x),                     \
+        reinterpret_cast<const uint4*>(Wr), H / 8, E, logits, k, mode, scores, idx64, idx32)
+    if (dtype == MOE_DTYPE_F16) { if (E <= 8) MOE_RT_LAUNCH(true, 8); else if (E <= 16) MOE_RT_LAUNCH(true, 16); else MOE_RT_LAUNCH(true, 32); }
+    else { if (E <= 8) MOE_RT_LAUNCH(false, 8); else if (E <= 16) MOE_RT_LAUNCH(false, 16); else MOE_RT_LAUNCH(false, 32); }
+#undef MOE_RT_LAUNCH
+    MOE_CHECK_LAUNCH("router_token_kernel");
+    return MOE_OK;
+  }
+  // one CTA per SM at most: every CTA stages the whole router weight
   int64_t blocks = ceil_div64(T, 8);      // a token per warp while the SMs last
   if (blocks > dev.sm_count) blocks = dev.sm_count;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define MOE_RL_LAUNCH(F16_, EMAX_)                                                                                       \
   do {                                                                                                                   \
     if (smem > 48 * 1024)                                                                                                \
