@@ -3,8 +3,11 @@
 // warp-private shared-memory histograms, no host round trip.
 #include "common.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <mutex>
+
+namespace cg = cooperative_groups;
 
 namespace moe {
 
@@ -26,7 +29,8 @@ constexpr int64_t RSMALL_TABLE = 131072; // ... as long as the units x experts t
 __host__ __device__ inline bool route_small_units(int64_t n, int E) {
   return n <= RSMALL_MAX && ((n + RUNIT_SMALL - 1) / RUNIT_SMALL) * (int64_t)E <= RSMALL_TABLE;
 }
-constexpr int64_t RSINGLE_MAX = 4096;    // up to here (half of it with many experts) one CTA does the whole stage in one launch
+constexpr int RCL_MAX_ROUNDS = 8;                               // entries per thread of the one-launch kernel
+constexpr int64_t RCLUSTER_MAX = 8ll * 1024 * RCL_MAX_ROUNDS;   // up to here one cluster of CTAs does the whole stage
 constexpr int RWPB = 8;            // warps per CTA in the count / scatter kernels
 
 // Expert id of flat entry i; with an id_map (int32 [E]) the id is translated, e.g. to the
@@ -188,84 +192,110 @@ route_scatter_kernel(const void* __restrict__ ids, int is64, int64_t n, int E, c
   }
 }
 
-// Small inputs (n <= RSINGLE_MAX): the whole stage in one CTA and one launch.  Counts by shared-memory atomics, an
-// exclusive scan over the experts, then the stable permutation in rounds of 1024 consecutive entries: inside a
-// round an entry's place is its expert's running start + the entries of that expert in earlier warps of the round
-// (one count per warp and expert, written by the first lane of each match group) + its rank among equal ids of
-// its own warp.  Same results as the three-kernel path, two launches fewer on the latency-bound small layers.
+// Up to RCLUSTER_MAX entries: the whole stage in one launch of one cluster of 1 to 8 CTAs.  The list is cut into one run of
+// 1024 * ROUNDS entries per CTA and of 32 * ROUNDS per warp.  A warp walks its run once, 32 entries at a time: match.any
+// ranks equal ids, the warp's own count of the expert gives the entries before them, and the sum of both stays in a
+// register.  Then the counts are summed, over the warps of the CTA, over the CTAs of the cluster (distributed shared
+// memory) and over the experts, and every entry's place is three look-ups.  Same results as the three kernels above.
+// What bounds it: latency.  Measured inside a graph (us, one CTA up to 2048 or 4096 entries and three kernels above -> this):
+// n = 3072, E = 9 6.0 -> 5.1; 4096, 64 10.4 -> 5.7; 8192, 8 9.2 -> 4.6; 32768, 256 17.9 -> 11.4; 65536, 256 29.5 -> 20.1.
+template <int ROUNDS>
 __global__ void __launch_bounds__(1024)
-route_small_kernel(const void* __restrict__ ids, int is64, int n, int E, const int32_t* __restrict__ id_map,
-                   int32_t* __restrict__ counts, int32_t* __restrict__ offsets, int32_t* __restrict__ perm,
-                   int32_t* __restrict__ inv, int32_t* __restrict__ status, int kx) {
+route_cluster_kernel(const void* __restrict__ ids, int is64, int n, int E, const int32_t* __restrict__ id_map,
+                     int32_t* __restrict__ counts, int32_t* __restrict__ offsets, int32_t* __restrict__ perm,
+                     int32_t* __restrict__ inv, int32_t* __restrict__ status, int kx) {
   extern __shared__ int32_t sh[];
-  int32_t* base = sh;                 // [E]   counts, then the running start of every expert
-  int32_t* wcnt = sh + E;             // [32][E]
+  int32_t* total = sh;                // [E]     entries of this CTA, read by the others
+  int32_t* start = sh + E;            // [E]     place of this CTA's first entry of an expert
+  int32_t* wcnt = sh + 2 * E;         // [32][E] entries per warp, then those of the warps before it
   __shared__ int32_t warp_tot[32];
-  __shared__ int32_t carry_s;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
-  for (int i = tid; i < 33 * E; i += 1024) sh[i] = 0;
-  if (tid == 0) carry_s = 0;
+  int nw = (n - crank * 1024 * ROUNDS + 32 * ROUNDS - 1) / (32 * ROUNDS);     // warps of this CTA that have entries
+  nw = nw < 0 ? 0 : (nw > 32 ? 32 : nw);
+  for (int i = tid; i < nw * E; i += 1024) wcnt[i] = 0;
   pdl_wait();
   pdl_trigger();
-  __syncthreads();
-  // a thread owns entries tid, tid + 1024, ...: at most RSINGLE_MAX / 1024 of them, kept in registers for the
-  // permutation rounds below (the loads are independent, so they are all in flight together)
-  constexpr int ROUNDS = RSINGLE_MAX / 1024;
-  int32_t ereg[ROUNDS];
+  const int first = (crank * 1024 + w * 32) * ROUNDS + lane;   // this lane's entries: first, first + 32, ...
+  int32_t e[ROUNDS], pos[ROUNDS];
   bool bad = false;
 #pragma unroll
   for (int r = 0; r < ROUNDS; ++r) {
-    const int i = r * 1024 + tid;
-    ereg[r] = i < n ? load_id(ids, is64, i, id_map, E, kx) : -1;
-    if (i < n && ereg[r] < 0) bad = true;
+    const int i = first + r * 32;
+    e[r] = i < n ? load_id(ids, is64, i, id_map, E, kx) : -1;
+    if (i < n && e[r] < 0) bad = true;
   }
-#pragma unroll
-  for (int r = 0; r < ROUNDS; ++r)
-    if (ereg[r] >= 0) atomicAdd(&base[ereg[r]], 1);
   if (bad && status) status[0] = ST_BAD_EXPERT_ID;
   __syncthreads();
-  for (int b0 = 0; b0 < E; b0 += 1024) {          // exclusive scan, 1024 experts at a time
-    const int e = b0 + tid;
-    const int32_t total = e < E ? base[e] : 0;
-    int32_t inc = total;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-      if (lane >= o) inc += v;
-    }
-    if (lane == 31) warp_tot[w] = inc;
-    __syncthreads();
-    int32_t before = carry_s;
-    for (int w2 = 0; w2 < w; ++w2) before += warp_tot[w2];
-    const int32_t start = before + inc - total;
-    if (e < E) { counts[e] = total; offsets[e] = start; base[e] = start; }
-    __syncthreads();
-    if (tid == 1023) carry_s = before + inc;
-    __syncthreads();
-  }
-  if (tid == 0) offsets[E] = carry_s;
-  if (!perm && !inv) return;
+  int32_t* wh = wcnt + w * E;
 #pragma unroll
   for (int r = 0; r < ROUNDS; ++r) {
-    if (r * 1024 >= n) break;
-    const int i = r * 1024 + tid;
-    const int e = ereg[r];
-    const bool valid = e >= 0;
-    const unsigned grp = __match_any_sync(0xFFFFFFFFu, valid ? (unsigned)e : (0x80000000u | (unsigned)lane));
+    const bool valid = e[r] >= 0;
+    // lanes without a valid id get a private group so that they match nobody
+    const unsigned grp = __match_any_sync(0xFFFFFFFFu, valid ? (unsigned)e[r] : (0x80000000u | (unsigned)lane));
     const int rank = __popc(grp & lt_mask);
-    if (valid && rank == 0) wcnt[w * E + e] = __popc(grp);
-    __syncthreads();
-    if (valid) {
-      int32_t pos = base[e] + rank;
-      for (int w2 = 0; w2 < w; ++w2) pos += wcnt[w2 * E + e];
-      if (perm) perm[pos] = i;
-      if (inv) inv[i] = pos;
-    }
-    __syncthreads();
-    if (valid && rank == 0) { atomicAdd(&base[e], __popc(grp)); wcnt[w * E + e] = 0; }
-    __syncthreads();
+    const int32_t base = valid ? wh[e[r]] : 0;
+    pos[r] = base + rank;
+    __syncwarp();
+    if (valid && rank == 0) wh[e[r]] = base + __popc(grp);
+    __syncwarp();
   }
+  __syncthreads();
+  int32_t own = 0;                    // thread x: expert x (E <= 1024)
+  if (tid < E) {
+#pragma unroll 8
+    for (int q = 0; q < nw; ++q) {
+      const int32_t v = wcnt[q * E + tid];
+      wcnt[q * E + tid] = own;
+      own += v;
+    }
+    total[tid] = own;
+  }
+  int32_t all = own, ahead = 0;       // entries of the expert in the whole list, and in the CTAs before this one
+  if (C > 1) cluster.sync();
+  if (C > 1 && tid < E) {
+    all = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      if (c < C) {
+        const int32_t v = cluster.map_shared_rank(total, c)[tid];
+        all += v;
+        if (c < crank) ahead += v;
+      }
+    }
+  }
+  int32_t inc = all;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  if (lane == 31) warp_tot[w] = inc;
+  __syncthreads();
+  int32_t before = 0;
+#pragma unroll
+  for (int q = 0; q < 32; ++q) before += q < w ? warp_tot[q] : 0;
+  const int32_t begin = before + inc - all;
+  if (tid < E) {
+    start[tid] = begin + ahead;
+    if (crank == 0) { counts[tid] = all; offsets[tid] = begin; }
+  }
+  if (crank == 0 && tid == 1023) offsets[E] = before + inc;
+  __syncthreads();
+  if (perm || inv) {
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+      if (e[r] >= 0) {
+        const int i = first + r * 32;
+        const int32_t place = start[e[r]] + wh[e[r]] + pos[r];
+        if (perm) perm[place] = i;
+        if (inv) inv[i] = place;
+      }
+    }
+  }
+  if (C > 1) cluster.sync();          // nobody leaves while its totals are still read
 }
 
 // ------------------------------------------------------------------------------------
@@ -656,22 +686,37 @@ int moe::route_histogram_ex(const void* topk_idx, int idx_is_int64, int64_t n, i
   if (need > 0 && (!ws || ws_bytes < need)) return fail(MOE_ERR_WORKSPACE, "route_histogram: workspace %zu < %zu", ws_bytes, need);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const bool small = route_small_units(n, E);
-  // MOE_B200_ROUTE_SINGLE_MAX moves the size up to which one CTA does the whole stage (for measurements; at most RSMALL_MAX)
+  // MOE_B200_ROUTE_SINGLE_MAX moves the size up to which one launch does the whole stage (for measurements; at most RCLUSTER_MAX)
   static const int64_t single_max = [] {
     const char* v = getenv("MOE_B200_ROUTE_SINGLE_MAX");
-    const int64_t m = v ? atoll(v) : RSINGLE_MAX;
-    return m < RSINGLE_MAX ? m : RSINGLE_MAX;
+    const int64_t m = v ? atoll(v) : RCLUSTER_MAX;
+    return m < RCLUSTER_MAX ? m : RCLUSTER_MAX;
   }();
-  // measured inside a CUDA graph (us, one CTA / three kernels): E = 256: n = 2048 8.9 / 7.0, 4096 14.2 / 8.4, 16384
-  // 45.6 / 13.6; E = 9: 3072 7.4 / 7.3, 4096 8.7 / 7.8, 16384 23.9 / 14.2.  One launch instead of three is worth
-  // a few microseconds of host time outside a graph, so the single CTA keeps the smallest inputs only.
-  const bool single = n <= single_max && (n <= RSINGLE_MAX / 2 || E <= 64);
-  if (single && n > 0 && E <= 1024) {   // one CTA, one launch
-    const size_t smem1 = (size_t)33 * E * 4;
+  if (n <= single_max && n > 0 && E <= 1024) {
+    // as many CTAs as give every thread one entry; above 8192 entries more entries per thread
+    int C = 1;
+    while (C < 8 && n > C * 1024) C <<= 1;
+    auto kernel = n <= C * 1024 ? route_cluster_kernel<1> : (n <= C * 2048 ? route_cluster_kernel<2>
+                : (n <= C * 4096 ? route_cluster_kernel<4> : route_cluster_kernel<RCL_MAX_ROUNDS>));
+    const size_t smem1 = (size_t)34 * E * 4;
     if (smem1 > 48 * 1024)
-      MOE_CUDA_CHECK(cudaFuncSetAttribute(route_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
-    MOE_LAUNCH("route_small_kernel", route_small_kernel, 1u, 1024u, smem1, st, pdl, topk_idx, idx_is_int64, (int)n, E, id_map,
-               counts, offsets, perm, inv, status, kx);
+      MOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 34 * 1024 * 4));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)C, 1, 1);
+    cfg.blockDim = dim3(1024, 1, 1);
+    cfg.dynamicSmemBytes = smem1;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 2 : 1;
+    MOE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, topk_idx, idx_is_int64, (int)n, E, id_map, counts, offsets, perm, inv,
+                                      status, kx));
     return MOE_OK;
   }
   const int64_t units = ceil_div64(n, small ? RUNIT_SMALL : RUNIT);
