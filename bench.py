@@ -359,10 +359,10 @@ def run_ours(args, wl_name, cfg):
             out_pin.copy_(step(), non_blocking=True)
 
         # kernels per layer.  Shared expert of the routed width and H % 64 == 0 (this workload): router GEMV with its
-        # top-k, histogram (one kernel for n <= 4096 entries with few experts, else three), up GEMM (gathers its rows,
+        # top-k, histogram (one kernel up to 65536 entries and 1024 experts, else three), up GEMM (gathers its rows,
         # shared expert as one more group), down GEMM, combine.  Otherwise: + row gather, + shared up and shared down.
         n1 = T * (k + S)
-        hist = 1 if (n1 <= 2048 or (n1 <= 4096 and E + S <= 64)) else 3
+        hist = 1 if n1 <= 65536 and E + S <= 1024 else 3
         ride = S == 1 and H % 64 == 0
         launches_per_step = 1 + hist + 2 + 1 + (0 if ride else (2 * (S > 0) + (H % 64 != 0)))
         tokens_per_step = T
@@ -381,7 +381,8 @@ def run_ours(args, wl_name, cfg):
             scores, idx32 = ops.topk_softmax(logits, k, mode="A", index_dtype=torch.int32)
             return layer.routed_forward(x, scores, idx32, Wg, Wu, Wd, ws, timers=timers)
 
-        launches_per_step = 7 if ws.fused_gather else 8   # topk, 3 x histogram, [gather,] up, down, combine
+        hist = 1 if T * k <= 65536 and E <= 1024 else 3
+        launches_per_step = 4 + hist + (0 if ws.fused_gather else 1)   # topk, histogram, [gather,] up, down, combine
         x_pin = x_cpu.pin_memory()
         lg_pin = logits_cpu.pin_memory()
         out_pin = torch.empty(T, H, dtype=torch.bfloat16).pin_memory()
@@ -774,7 +775,7 @@ def router_block(dev, peaks, flush, with_cpu):
 
 def c2_block(dev, peaks, flush, with_cpu):
     """Grouped expert GEMM of the contract: T=4096 tokens, top-2 of E=8, X [4096,1024] . W[e] [256,1024]^T, bf16.
-    `us_api` is kernels.grouped_gemm (histogram + row gather + tcgen05 GEMM + un-sort scatter, 5 launches);
+    `us_api` is kernels.grouped_gemm (histogram, then the tcgen05 GEMM with row gather and un-sort scatter: 2 launches);
     `us_gemm` the GEMM launch alone on rows already sorted by expert."""
     from tilelang_moe_b200 import kernels, ops
     c = C2
