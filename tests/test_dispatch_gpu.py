@@ -89,3 +89,29 @@ def test_few_experts_a_cta_or_a_warp_per_token(cuda, lib, T, H, E, k, dtype):
         s_ref, i_ref = O.topk_softmax(lg.cpu(), k, mode)
         assert torch.equal(i.cpu(), i_ref)
         torch.testing.assert_close(s.cpu(), s_ref, rtol=1e-6, atol=1e-30)
+
+
+@pytest.mark.parametrize("T,H,I,E,k,shared", [(1, 64, 8, 4, 2, 0), (5, 192, 40, 8, 2, 1), (31, 256, 512, 8, 2, 1), (32, 2048, 512, 8, 2, 1),
+                                              (32, 320, 264, 16, 8, 0), (33, 2048, 512, 8, 2, 1), (20, 1024, 136, 6, 6, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_up_gemm_of_few_rows(cuda, lib, T, H, I, E, k, shared, dtype):
+    """Up to 32 tokens the layer's up GEMM holds 32 rows of A per stage: the same bits as the wide tiles that the stage-by-stage
+    layer takes (it does not bound the rows of a group), and close to the oracle."""
+    from tilelang_moe_b200 import kernels, layer
+    x, w = O.make_fusedmoe_inputs(1, T, H, I, E, shared, k, dtype=dtype, seed=T + I)
+    names = ["router_weight", "shared_gate", "shared_up", "shared_down", "routed_gate", "routed_up", "routed_down"]
+    ws = [w[n].to(cuda) if shared or not n.startswith("shared") else None for n in names]
+    lg = O.router_logits(x.view(-1, H), w["router_weight"])
+    m = kernels.FusedMoETileLang(H, I, E, shared, k, 1, T, dtype=dtype)
+    y = m.forward(x.to(cuda), *ws, logits=lg.to(cuda))
+    ref = layer.moe_forward(x.to(cuda), *ws, k, logits=lg.to(cuda))
+    ops.check_status(cuda)
+    assert torch.equal(y, ref)
+    n = min(T, 32)                        # one expert list of at most 32 rows through the generic entry point
+    ids = torch.randint(0, E, (n, 1), generator=torch.Generator().manual_seed(T))
+    _, offs, perm, _ = O.route_histogram(ids, E)
+    xs = x.view(-1, H)[:n]
+    act = ops.grouped_gemm_sorted(ops.GEMM_SILU_GATE, xs.to(cuda), ws[4], offs.to(cuda), B2=ws[5], gather=perm.to(cuda))
+    plain = ops.grouped_gemm_sorted(ops.GEMM_SILU_GATE, xs[perm.long()].to(cuda), ws[4], offs.to(cuda), B2=ws[5])
+    ops.check_status(cuda)
+    assert torch.equal(act, plain)

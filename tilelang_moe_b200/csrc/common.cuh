@@ -180,11 +180,12 @@ int grouped_gemm_scatter_slots(const void* A, const void* B, const int32_t* offs
                                const float* row_w, int w_slots, void* Y, int64_t ldy, int64_t max_rows, int K, int N, int E,
                                int dtype, int32_t* status, void* stream, bool pdl);
 
-// the public grouped GEMMs and the combine behind another kernel of the same call (pdl: see above; gemm_sm100.cu, route.cu)
+// the public grouped GEMMs and the combine behind another kernel of the same call (pdl: see above; gemm_sm100.cu, route.cu);
+// group_rows > 0: the caller knows that no group has more rows
 int grouped_gemm_gathered_ex(int epilogue, const void* X, int64_t x_rows, const int32_t* gather_idx, int gather_div,
                              const void* B, const void* B2, const int32_t* offsets, const int32_t* dst_rows,
                              const float* row_w, void* Y, int64_t ldy, int64_t max_rows, int64_t expected_rows, int K, int N,
-                             int E, int dtype, int32_t* status, void* stream, bool pdl);
+                             int E, int dtype, int32_t* status, void* stream, bool pdl, int64_t group_rows = 0);
 int grouped_gemm_ex(int epilogue, const void* A, const void* B, const void* B2, const int32_t* offsets,
                     const int32_t* dst_rows, const float* row_w, void* Y, int64_t ldy, int64_t max_rows,
                     int64_t expected_rows, int K, int N, int E, int dtype, int32_t* status, void* stream, bool pdl);

@@ -70,18 +70,23 @@ constexpr int MAX_E = 1024;
 constexpr uint64_t WAIT_LIMIT_NS = 1000ull * 1000ull * 1000ull;   // 1 s per barrier wait
 constexpr uint64_t DRAIN_LIMIT_NS = 20ull * 1000ull * 1000ull;    // 20 ms when draining after a failure
 
-template <int MT, int BN>
+// AR: rows of A a stage holds.  128, or 32 for groups of at most 32 rows: their M = 64 instructions read 64 rows, the
+// upper half from whatever follows in the stage, and nothing of what they make of it is stored.
+template <int MT, int BN, int AR = BM>
 struct Cfg {
-  static constexpr int A_HALF_BYTES = BM * BK * 2;         // one 128-row A tile
+  static constexpr int A_HALF_BYTES = AR * BK * 2;         // one A tile
   static constexpr int A_BYTES = MT * A_HALF_BYTES;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (192 * 1024) / STAGE_BYTES;  // 6, 4 or 3
+  static constexpr int STAGES = (192 * 1024) / STAGE_BYTES;  // 6, 4 or 3; with 32 rows of A 16, 9 or 5
   static constexpr int ACC_BUFS = (MT * BN * 2 <= 512) ? 2 : 1;
-  static constexpr int TMEM_COLS = ACC_BUFS * MT * BN;       // 256 or 512: powers of two >= 32
-  // layout: [stages][barriers 256 B][tile tables]
+  static constexpr int TMEM_COLS = ACC_BUFS * MT * BN;       // 128, 256 or 512: powers of two >= 32
+  static_assert(AR == BM || A_HALF_BYTES + B_BYTES >= 64 * BK * 2, "an M = 64 instruction stays inside its stage");
+  // layout: [stages][barriers, tensor-memory slot and abort flag 384 B][tile tables]
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
-  static constexpr int TABLE_OFFSET = BAR_OFFSET + 256;
+  static constexpr int SLOT_OFFSET = BAR_OFFSET + 320;
+  static_assert((2 * STAGES + 5) * 8 <= 320, "barriers fit below the tensor-memory slot");
+  static constexpr int TABLE_OFFSET = BAR_OFFSET + 384;
   static constexpr int STAGING_OFFSET = (TABLE_OFFSET + 3 * (MAX_E + 1) * 4 + 127) & ~127;   // 16-byte accesses
   static constexpr int SMEM_BYTES = STAGING_OFFSET + 1024;  // + alignment slack
   // 16-bit rows: 4 warps x 32 rows x (128 B + 16 B pad) to turn per-thread rows into 128-byte row segments;
@@ -570,11 +575,11 @@ __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t ta
 }
 
 // ------------------------------------------------------------------------------ kernel
-template <int MT, int BN, int EPI, bool GATHER>
+template <int MT, int BN, int EPI, bool GATHER, int AR>
 __global__ void __launch_bounds__(GATHER ? NUM_THREADS_GATHER : NUM_THREADS, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmB2, const Params p) {
-  using C = Cfg<MT, BN>;
+  using C = Cfg<MT, BN, AR>;
   constexpr int STAGES = C::STAGES;
   constexpr int ACC_BUFS = C::ACC_BUFS;
   constexpr int TILE_ROWS = MT * BM;
@@ -584,8 +589,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::BAR_OFFSET);
   // bars[0..S) full, [S..2S) empty, [2S..2S+2) tmem_full, [2S+2..2S+4) tmem_empty, [2S+4] drain
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::BAR_OFFSET + 200);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::BAR_OFFSET + 208);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::SLOT_OFFSET);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::SLOT_OFFSET + 8);
   int32_t* tstart = reinterpret_cast<int32_t*>(smem + C::TABLE_OFFSET);
   int32_t* offs = tstart + (MAX_E + 1);
   int32_t* lstart = offs + (MAX_E + 1);            // mixed schedule: tstart then counts the heavy experts' tiles only
@@ -600,8 +605,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   // ---- set-up: barriers, TMEM, tile table
   if (threadIdx.x == 0) {
-    // full: the TMA producer's arrive (+ one arrival per lane of the two gather warps once its copies have landed)
-    for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, gather ? 65 : 1); mbar_init(empty0 + 8 * s, 1); }
+    // full: the TMA producer's arrive (+ one arrival per lane of the gather warps, one of them for 32 rows, once its
+    // copies have landed)
+    for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, gather ? (AR == BM ? 65 : 33) : 1); mbar_init(empty0 + 8 * s, 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, 4); }
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
@@ -726,7 +732,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // ===================================================================== A-row gather (only when asked to)
     // Two warps, 64 tile rows each.  8 lanes cover the 128 bytes of one row, so one cp.async instruction moves
     // four whole 128-byte row pieces; a lane keeps the 16 source pointers it needs for the whole tile.
-    if (gather) {
+    constexpr int GROUPS = AR == BM ? 16 : AR / 4;       // groups of four rows per warp
+    if (gather && (AR == BM || warp == 6)) {
       const unsigned char* src_base = reinterpret_cast<const unsigned char*>(p.a_src);
       const size_t row_bytes = (size_t)p.K * 2;
       const int chunk = lane & 7, sub = lane >> 3;
@@ -751,10 +758,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           }
           src_row[s] = v;
         }
-        const unsigned char* rp[16];
+        const unsigned char* rp[GROUPS];
         uint32_t live = 0;                                                  // bit `it`: that row belongs to the group
 #pragma unroll
-        for (int it = 0; it < 16; ++it) {
+        for (int it = 0; it < GROUPS; ++it) {
           const int row = it * 4 + sub;                                     // row within this warp's half
           const uint32_t sr = __shfl_sync(0xFFFFFFFFu, src_row[it >> 3], row & 31);
           rp[it] = src_base + (size_t)sr * row_bytes + chunk * 16;
@@ -765,7 +772,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           const uint32_t sa = smem_u32(smem + stage * C::STAGE_BYTES) + half_row0 * 128;
           const size_t koff = (size_t)kb * (BK * 2);
 #pragma unroll
-          for (int it = 0; it < 16; ++it) {
+          for (int it = 0; it < GROUPS; ++it) {
             const int row = it * 4 + sub;
             // 128-byte swizzle: 16-byte chunk c of row r sits at chunk (c ^ (r & 7)) of that row
             cp_async_16(sa + row * 128 + ((chunk ^ (row & 7)) << 4), rp[it] + koff, (live >> it) & 1u ? 16u : 0u);
@@ -1396,15 +1403,15 @@ static int allow_dynamic_smem(Kernel kernel, int bytes, std::atomic<bool>* done_
   return MOE_OK;
 }
 
-template <int MT, int BN, int EPI, bool GATHER>
+template <int MT, int BN, int EPI, bool GATHER, int AR = BM>
 static int launch_g(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2, const Params& p, int grid,
                     cudaStream_t st) {
-  using C = Cfg<MT, BN>;
+  using C = Cfg<MT, BN, AR>;
   constexpr int SMEM = EPI == MOE_GEMM_PLAIN_F32 || EPI == MOE_GEMM_SILU_GATE ? C::SMEM_BYTES : C::SMEM_BYTES_STAGED;
   static std::atomic<bool> attr_set[64];
-  int rc = allow_dynamic_smem(grouped_gemm_kernel<MT, BN, EPI, GATHER>, SMEM, attr_set);
+  int rc = allow_dynamic_smem(grouped_gemm_kernel<MT, BN, EPI, GATHER, AR>, SMEM, attr_set);
   if (rc) return rc;
-  MOE_LAUNCH("grouped_gemm_kernel", grouped_gemm_kernel<MT, BN, EPI, GATHER>, (unsigned)grid,
+  MOE_LAUNCH("grouped_gemm_kernel", grouped_gemm_kernel<MT, BN, EPI, GATHER, AR>, (unsigned)grid,
              GATHER ? NUM_THREADS_GATHER : NUM_THREADS, SMEM, st, p.pdl != 0, tA, tB, tB2, p);
   return MOE_OK;
 }
@@ -1438,6 +1445,7 @@ struct GatherArgs {           // A rows fetched through an index list instead of
   int64_t dense_rows = 0;     // > 0 with offsets == nullptr: one group of this many rows (E must be 1)
   int w_slots = 0;            // see Params::w_slots
   bool pdl = false;           // behind another kernel of the same library call
+  int64_t group_rows = 0;     // > 0: no group has more rows than this
 };
 
 static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const void* B2, const int32_t* offsets,
@@ -1465,13 +1473,13 @@ extern "C" int moe_grouped_gemm(int epilogue, const void* A, const void* B, cons
 int moe::grouped_gemm_gathered_ex(int epilogue, const void* X, int64_t x_rows, const int32_t* gather_idx, int gather_div,
                                   const void* B, const void* B2, const int32_t* offsets, const int32_t* dst_rows,
                                   const float* row_w, void* Y, int64_t ldy, int64_t max_rows, int64_t expected_rows, int K,
-                                  int N, int E, int dtype, int32_t* status, void* stream, bool pdl) {
+                                  int N, int E, int dtype, int32_t* status, void* stream, bool pdl, int64_t group_rows) {
   if (!gather_idx) return fail(MOE_ERR_ARG, "grouped_gemm_gathered: null index list");
   if (gather_div < 1 || x_rows < 1 || x_rows > 0x7FFFFFFFll)
     return fail(MOE_ERR_ARG, "grouped_gemm_gathered: bad gather_div=%d or x_rows=%lld", gather_div, (long long)x_rows);
   if (K % 64) return fail(MOE_ERR_UNSUPPORTED, "grouped_gemm_gathered: K=%d must be a multiple of 64", K);
   GatherArgs ga;
-  ga.idx = gather_idx; ga.div = gather_div; ga.src_rows = x_rows; ga.pdl = pdl;
+  ga.idx = gather_idx; ga.div = gather_div; ga.src_rows = x_rows; ga.pdl = pdl; ga.group_rows = group_rows;
   return grouped_gemm_impl(epilogue, X, B, B2, offsets, dst_rows, row_w, Y, ldy, max_rows, K, N, E, status, stream,
                            nullptr, nullptr, 0, expected_rows, dtype, ga);
 }
@@ -1660,6 +1668,13 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
     if (force[0] == 'p') pair = pair_ok;
     else if (atoi(force) == 128) pair = false;
   }
+  // Groups of at most 32 rows that leave most SMs without a 256-column tile: 64-column tiles spread the weights over more
+  // SMs, and with 32 rows of A per stage nearly the whole ring holds weights in flight, which is what bounds their stream.
+  // Measured: a decode step of 8 tokens through 8 + 1 experts, H = 2048, I = 512 36.9 -> 34.9 us; 64-column tiles with 128
+  // rows of A per stage were no faster than 256-column ones (8 KB of weights in a 24 KB stage).
+  const int64_t group_rows = ga.group_rows > 0 && ga.group_rows < max_rows ? ga.group_rows : max_rows;
+  const bool few_rows = gate && ga.idx && group_rows <= 32 && (live_rows < E ? live_rows : E) * n_tiles_256 * 2 <= dev.sm_count;
+  if (few_rows) BN = 64;
   const int out_cols = gate ? BN / 2 : BN;
 
   Params p;
@@ -1684,7 +1699,7 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
   // measured on the DeepSeek-V3-shaped layer, ten alternating runs of 20 steps: 7.56 -> 7.29 ms per step (-3.6 %) and the
   // median SM clock of the power-capped steps back at its maximum; MOE_B200_M64=0 switches it off for such comparisons
   static const int env_m64 = [] { const char* h = getenv("MOE_B200_M64"); return h ? atoi(h) : 1; }();
-  p.m64 = env_m64;
+  p.m64 = env_m64 || few_rows;
   p.l2_hints = env_hints;
   p.mixed = env_mixed && offsets != nullptr;
 
@@ -1742,7 +1757,9 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
     case MOE_GEMM_PLAIN: MOE_GEMM_CASE(MOE_GEMM_PLAIN);
     case MOE_GEMM_SCALE_SCATTER: MOE_GEMM_CASE(MOE_GEMM_SCALE_SCATTER);
     case MOE_GEMM_PLAIN_F32: MOE_GEMM_CASE(MOE_GEMM_PLAIN_F32);
-    default: return launch<1, 256, MOE_GEMM_SILU_GATE>(tA, tB, tB2, p, grid, st);
+    default:
+      if (few_rows) return launch_g<1, 64, MOE_GEMM_SILU_GATE, true, 32>(tA, tB, tB2, p, grid, st);
+      return launch<1, 256, MOE_GEMM_SILU_GATE>(tA, tB, tB2, p, grid, st);
   }
 #undef MOE_GEMM_CASE
 }

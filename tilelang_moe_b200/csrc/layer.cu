@@ -227,7 +227,7 @@ routed:
                             moe_route_histogram_workspace(n1, E + 1), status, stream, k, pdl);
     if (rc) return rc;
     rc = grouped_gemm_gathered_ex(MOE_GEMM_SILU_GATE, x, T, perm, k + 1, routed_gate, routed_up, offsets, nullptr, nullptr, act,
-                                   I, n1, 0, H, I, E + 1, dtype, status, stream, pdl);
+                                   I, n1, 0, H, I, E + 1, dtype, status, stream, pdl, T);
     if (rc) return rc;
     rc = grouped_gemm_scatter_slots(act, routed_down, offsets, perm, scores, k, yk, H, n1, I, H, E + 1, dtype, status, stream, pdl);
     if (rc) return rc;
@@ -238,7 +238,7 @@ routed:
   if (rc) return leave(rc);
   if (H % 64 == 0) {
     rc = grouped_gemm_gathered_ex(MOE_GEMM_SILU_GATE, x, T, perm, k, routed_gate, routed_up, offsets, nullptr, nullptr, act, I,
-                                  n, 0, H, I, E, dtype, status, stream, pdl);
+                                  n, 0, H, I, E, dtype, status, stream, pdl, T);
     if (rc) return leave(rc);
     rc = grouped_gemm_ex(MOE_GEMM_SCALE_SCATTER_DSTW, act, routed_down, nullptr, offsets, perm, scores, yk, H, n, 0, I, H, E,
                          dtype, status, stream, pdl);
