@@ -29,7 +29,7 @@ def _rows(kind, M, N, g):
 
 
 @pytest.mark.parametrize("kind", ["normal", "ties", "const", "sorted", "masked", "nan"])
-@pytest.mark.parametrize("N", [8, 12, 32, 36, 64, 68, 128, 132, 256, 260, 512, 516, 1000, 1024])
+@pytest.mark.parametrize("N", [8, 12, 32, 36, 64, 68, 72, 128, 132, 256, 260, 512, 516, 1000, 1024])
 def test_group_and_lane_kernels(cuda, lib, N, kind):
     M = 2051 if N <= 256 else 83     # the last warp's rows run past the end
     g = torch.Generator().manual_seed(N)

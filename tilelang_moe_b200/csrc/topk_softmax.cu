@@ -145,8 +145,8 @@ static int launch_warp(const float* logits, int64_t M, int N, int64_t ld, int k,
 //
 // L = 4 .. 32 neighbouring lanes share a row, EPT = 8 .. 32 logits per lane, straight from global memory into registers
 // with 16-byte loads (the only pass over the logits).  A row is never ordered as a whole:
-//   1. every lane takes the maxima of four parts of its logits; the group merges them over shuffles (sorted lists, the
-//      upper half kept) into V, the K-th largest of the 4 * L part maxima - a lower bound of the K-th largest logit;
+//   1. every lane takes the maxima of four parts of its logits, strided over the row; the group merges them over shuffles
+//      (sorted lists, the upper half kept) into V, the K-th largest of the 4 * L part maxima - a lower bound of the K-th largest logit;
 //   2. the logits not below V, seven or eight of them as a rule, are collected in shared memory as 64-bit key | column
 //      entries (equal keys: lowest column first);
 //   3. each lane ranks its share of them against all of them; the entries of rank < k are the result, in order.
@@ -185,7 +185,6 @@ topk_group_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
   constexpr int CAP = L == 32 ? 32 : 16;            // entries a row may collect
   constexpr int HELD = CAP / L;                     // entries a lane ranks
   constexpr int P = K > 4 ? 8 : (K > 2 ? 4 : 2);    // length of the merged lists of maxima
-  constexpr int PART = EPT / 4;
   __shared__ uint64_t cand_s[GROUP_WARPS][RPW][CAP + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane & (L - 1), rw = lane / L;
@@ -213,13 +212,14 @@ topk_group_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
     }
   }
 
-  // ---- 1. V
+  // ---- 1. V.  Part q of a lane holds the q-th logits of all its vectors: parts are equally long for every N, and a masked
+  //      run of columns takes as much from each
   float g[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     float m = NEG_INF;
 #pragma unroll
-    for (int j = 0; j < PART; ++j) m = fmaxf(m, x[q * PART + j]);
+    for (int i = 0; i < EPT / 4; ++i) m = fmaxf(m, x[4 * i + q]);
     g[q] = m;
   }
   ce_desc(g[0], g[1]); ce_desc(g[2], g[3]); ce_desc(g[0], g[2]); ce_desc(g[1], g[3]); ce_desc(g[1], g[2]);
