@@ -55,3 +55,15 @@ def test_padded_rows_and_both_index_types(cuda, lib):
         s_ref, i_ref = O.topk_softmax(view.cpu(), 5)
         assert torch.equal(i64.cpu(), i_ref) and torch.equal(i32.cpu().long(), i_ref)
         torch.testing.assert_close(s.cpu(), s_ref, rtol=RTOL, atol=1e-30)
+
+
+def test_large_row_counts_take_fewer_lanes_per_row(cuda, lib):
+    x = torch.randn(262145, 68, device=cuda, generator=torch.Generator(device=cuda).manual_seed(2))
+    s, i = ops.topk_softmax(x, 8)                     # four lanes per row
+    s1, i1 = ops.topk_softmax(x[:262144], 8)          # eight
+    assert torch.equal(i[:-1], i1)
+    torch.testing.assert_close(s[:-1], s1, rtol=2 * RTOL, atol=1e-30)   # two kernels, each within RTOL of the exact scores
+    rows = torch.arange(0, 262145, 997)
+    s_ref, i_ref = O.topk_softmax(x[rows.to(cuda)].cpu(), 8)
+    assert torch.equal(i[rows.to(cuda)].cpu(), i_ref)
+    torch.testing.assert_close(s[rows.to(cuda)].cpu(), s_ref, rtol=RTOL, atol=1e-30)

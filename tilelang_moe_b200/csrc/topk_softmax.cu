@@ -1036,6 +1036,8 @@ extern "C" int moe_topk_softmax(const float* logits, int64_t M, int64_t N, int64
   // Measured (us): 320 rows of 128, k = 6: a warp per row 2.5, lane groups 3.5; of 256, k = 8: 3.2, 3.3; of 512: 4.0, 3.3;
   // of 1024: 5.8, 3.4.  2048 rows of 16: a lane per row 2.5, lane groups 2.5; 8192: 2.6, 2.6; 32768: 2.9, 3.8; rows of 64
   // (a lane per row is built for 32 at most): 32768 4.3, 4.5.
+  // k = 7, 8 of 65 to 128: four lanes have 16 parts, of which the 8th leaves some rows with more than 16 entries; eight lanes
+  // have 32 (2048 rows 3.1 against 6.3, 32768 9.2 against 13.0, 131072 27.5 against 28.9, 1048576 190 against 178).
   if (n <= 1024 && k <= 8 && n >= 8 && vec_rows && (M >= 2048 || n > 256)) {
     if (n <= LANE_NMAX) {
 #define MOE_LANE_CASE(K_) return launch_lane<K_>(logits, M, n, ld, k, mode, scores, indices, indices32, dev.sm_count, st)
@@ -1049,6 +1051,7 @@ extern "C" int moe_topk_softmax(const float* logits, int64_t M, int64_t N, int64
 #define MOE_GROUP_K(K_)                          \
   {                                              \
     if (n <= 64) MOE_GROUP_CASE(K_, 4, 16);      \
+    if (n <= 128 && K_ == 8 && M <= 262144) MOE_GROUP_CASE(K_, 8, 16); \
     if (n <= 128) MOE_GROUP_CASE(K_, 4, 32);     \
     if (n <= 256) MOE_GROUP_CASE(K_, 8, 32);     \
     if (n <= 512) MOE_GROUP_CASE(K_, 16, 32);    \
