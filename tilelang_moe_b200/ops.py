@@ -240,8 +240,12 @@ def grouped_gemm_routed(X: torch.Tensor, W: torch.Tensor, ids: torch.Tensor, k: 
     E, I, K2 = W.shape
     if K2 != H:
         raise ValueError(f"inner dimensions differ: X has K={H}, W has K={K2}")
-    ids = ids.contiguous()
+    if k < 0 or ids.numel() != T * k:      # the library reads T * k ids from the pointer
+        raise ValueError(f"{ids.numel()} expert ids for {T} rows of {k} experts each")
     dev = X.device
+    if W.device != dev or ids.device != dev:
+        raise ValueError(f"X, W and the expert ids must be on one device, not on {dev}, {W.device} and {ids.device}")
+    ids = ids.contiguous()
     lib = _lib.load()
     need = lib.moe_grouped_gemm_routed_workspace(T, k, H, E)
     ws = torch.empty(max(need, 4), dtype=torch.uint8, device=dev)
