@@ -244,6 +244,8 @@ int moe_grouped_gemm_routed(const void* X, int64_t T, int k, const void* ids, in
  * projection), the shared expert runs as expert E of the routed grouped GEMMs - every token gets k + 1 entries, the
  * last with weight 1 - and the whole layer is five launches on `stream` (the reference overlaps its shared and
  * routed kernels on two streams instead, kernels/fusedmoe_tilelang.py:428-553).  Same bits as the other form.
+ * moe_layer_forward_ex with shared_group = 1 asks for that form wherever the shared weights lie (they are read in place;
+ * MOE_ERR_ARG unless SI == I, H % 64 == 0 and E < 1024); with 0 it is moe_layer_forward.
  * The router kernel (one kernel, split along K, or GEMM then top-k) is chosen from T, H and E: fp32 logits of one
  * token can differ in summation order between batch sizes, so a near-tie may route differently in another batch size.
  */
@@ -253,6 +255,11 @@ int moe_layer_forward(const void* x, const void* router_weight, const float* log
                       const void* routed_up, const void* routed_down, int64_t T, int H, int I, int E, int k,
                       int SI, int dtype, void* ws, size_t ws_bytes, void* out, int32_t* status, void* stream,
                       void* side_stream);
+int moe_layer_forward_ex(const void* x, const void* router_weight, const float* logits, const void* shared_gate,
+                         const void* shared_up, const void* shared_down, const void* routed_gate,
+                         const void* routed_up, const void* routed_down, int64_t T, int H, int I, int E, int k,
+                         int SI, int dtype, void* ws, size_t ws_bytes, void* out, int32_t* status, void* stream,
+                         void* side_stream, int shared_group);
 
 /* ---- mHC pre / post blocks ---------------------------------------------------------------
  * The operators on either side of the MoE layer in the model the reference targets

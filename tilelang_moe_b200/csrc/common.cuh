@@ -178,14 +178,16 @@ int route_histogram_ex(const void* topk_idx, int idx_is_int64, int64_t n, int E,
 // first w_slots of a run read row_w[token * w_slots + slot], the last one (the shared expert's row) weighs 1 (gemm_sm100.cu)
 int grouped_gemm_scatter_slots(const void* A, const void* B, const int32_t* offsets, const int32_t* dst_rows,
                                const float* row_w, int w_slots, void* Y, int64_t ldy, int64_t max_rows, int K, int N, int E,
-                               int dtype, int32_t* status, void* stream, bool pdl);
+                               int dtype, int32_t* status, void* stream, bool pdl, const void* last_B);
 
 // the public grouped GEMMs and the combine behind another kernel of the same call (pdl: see above; gemm_sm100.cu, route.cu);
-// group_rows > 0: the caller knows that no group has more rows
+// group_rows > 0: the caller knows that no group has more rows; last_B (and last_B2 with B2), here and above: the weights
+// of group E - 1 lie there, those of the others in B [E - 1, N, K]
 int grouped_gemm_gathered_ex(int epilogue, const void* X, int64_t x_rows, const int32_t* gather_idx, int gather_div,
                              const void* B, const void* B2, const int32_t* offsets, const int32_t* dst_rows,
                              const float* row_w, void* Y, int64_t ldy, int64_t max_rows, int64_t expected_rows, int K, int N,
-                             int E, int dtype, int32_t* status, void* stream, bool pdl, int64_t group_rows = 0);
+                             int E, int dtype, int32_t* status, void* stream, bool pdl, int64_t group_rows = 0,
+                             const void* last_B = nullptr, const void* last_B2 = nullptr);
 int grouped_gemm_ex(int epilogue, const void* A, const void* B, const void* B2, const int32_t* offsets,
                     const int32_t* dst_rows, const float* row_w, void* Y, int64_t ldy, int64_t max_rows,
                     int64_t expected_rows, int K, int N, int E, int dtype, int32_t* status, void* stream, bool pdl);

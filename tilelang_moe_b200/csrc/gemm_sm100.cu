@@ -136,7 +136,14 @@ struct Params {
   int mixed = 0;           // 128-row kernel: single-tile and multi-tile experts interleaved in the tile order
   int m64 = 0;             // 128-row kernel: tiles with at most 64 live rows as M = 64 instructions
   int pdl = 0;             // host side: launched behind another kernel of the same call
+  int b_groups = MAX_E;    // groups from this one on (the last, if any) have their weights in a tensor of their own: WeightMap
   int64_t y_rows = 0;      // rows of Y when dst_rows scatters into it (the checked build compares every destination with it)
+};
+
+// Tensor maps of a weight: of the [E, N, K] tensor, and of the last group's [N, K] where that one lies elsewhere (the
+// shared expert of a layer beside its routed experts: two allocations of the caller's, read where they are).
+struct WeightMap {
+  CUtensorMap m[2];
 };
 
 // ------------------------------------------------------------------------------ PTX wrappers
@@ -577,8 +584,8 @@ __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t ta
 // ------------------------------------------------------------------------------ kernel
 template <int MT, int BN, int EPI, bool GATHER, int AR>
 __global__ void __launch_bounds__(GATHER ? NUM_THREADS_GATHER : NUM_THREADS, 1)
-grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    const __grid_constant__ CUtensorMap tmB2, const Params p) {
+grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ WeightMap tmB,
+                    const __grid_constant__ WeightMap tmB2, const Params p) {
   using C = Cfg<MT, BN, AR>;
   constexpr int STAGES = C::STAGES;
   constexpr int ACC_BUFS = C::ACC_BUFS;
@@ -613,8 +620,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     prefetch_tmap(&tmA);
-    prefetch_tmap(&tmB);
-    if (EPI == MOE_GEMM_SILU_GATE) prefetch_tmap(&tmB2);
+    prefetch_tmap(&tmB.m[0]);
+    if (EPI == MOE_GEMM_SILU_GATE) prefetch_tmap(&tmB2.m[0]);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
@@ -648,6 +655,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int k0 = p.ksplit ? t.n_tile * NKB * BK : 0;        // first K element of this tile's slice
       // weights of an expert with a single row tile are read exactly once: they should leave L2 first; weights that
       // several row tiles share stay as long as L2 lets them
+      const int own = t.e >= p.b_groups;                        // the group with a weight tensor of its own
+      const int e_b = own ? 0 : t.e;
       const uint64_t b_policy = p.l2_hints == 0 ? pol_normal : (t.m_tiles == 1 ? pol_first : (p.l2_hints == 2 ? pol_last : pol_normal));
       for (int kb = 0; kb < NKB; ++kb) {
         if (!mbar_wait(empty0 + 8 * stage, phase ^ 1, abort_flag, p.status, 1)) { ok = false; break; }
@@ -658,10 +667,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           mbar_arrive_expect_tx(full, gather ? p.b_tx_bytes : C::A_BYTES + p.b_tx_bytes);
           if (!gather) tma_load_2d(sa, &tmA, full, k0 + kb * BK, t.row0);
           if (EPI == MOE_GEMM_SILU_GATE) {
-            tma_load_3d_hint(sb, &tmB, full, kb * BK, n0, t.e, b_policy);
-            tma_load_3d_hint(sb + C::B_BYTES / 2, &tmB2, full, kb * BK, n0, t.e, b_policy);
+            tma_load_3d_hint(sb, &tmB.m[own], full, kb * BK, n0, e_b, b_policy);
+            tma_load_3d_hint(sb + C::B_BYTES / 2, &tmB2.m[own], full, kb * BK, n0, e_b, b_policy);
           } else {
-            tma_load_3d_hint(sb, &tmB, full, k0 + kb * BK, n0, t.e, b_policy);
+            tma_load_3d_hint(sb, &tmB.m[own], full, k0 + kb * BK, n0, e_b, b_policy);
           }
         }
         __syncwarp();
@@ -1069,7 +1078,7 @@ __device__ __forceinline__ void store_row_chunk(const Params& p, void* ybase, in
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA64,
-                         const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmB2,
+                         const __grid_constant__ WeightMap tmB, const __grid_constant__ WeightMap tmB2,
                          const Params p) {
   using C = PairCfg;
   constexpr int STAGES = C::STAGES;
@@ -1109,8 +1118,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmA64);
-    prefetch_tmap(&tmB);
-    if (GATE) prefetch_tmap(&tmB2);
+    prefetch_tmap(&tmB.m[0]);
+    if (GATE) prefetch_tmap(&tmB2.m[0]);
   }
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(tmem_slot), C::TMEM_COLS);
@@ -1138,6 +1147,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       const bool light = EPI != EPI_ROUTER && t.row_end - t.row0 <= BM;           // 128-row tile: 64 rows per CTA
       const int n0 = t.n_tile * OUT_COLS;
       const int a_row = t.row0 + (int)rank * (light ? BM / 2 : BM);
+      const int own = t.e >= p.b_groups;                     // the group with a weight tensor of its own
+      const int e_b = own ? 0 : t.e;
       const uint32_t tx = light ? 2u * (C::A_BYTES / 2 + C::B_BYTES) : 2u * C::STAGE_BYTES;
       // read by the MMA issuer after the first full barrier of the tile; the producer runs at most STAGES (< 8) k-blocks,
       // hence tiles, ahead of it
@@ -1152,10 +1163,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           if (leader) mbar_arrive_expect_tx(full0 + 8 * stage, tx);
           tma_load_2d_pair(sa, light ? &tmA64 : &tmA, lead_full, kb * BK, a_row);
           if (GATE) {   // this CTA's 64 gate rows, then its 64 up rows of the same output columns
-            tma_load_3d_pair(sb, &tmB, lead_full, kb * BK, n0 + (int)rank * (OUT_COLS / 2), t.e);
-            tma_load_3d_pair(sb + C::B_BYTES / 2, &tmB2, lead_full, kb * BK, n0 + (int)rank * (OUT_COLS / 2), t.e);
+            tma_load_3d_pair(sb, &tmB.m[own], lead_full, kb * BK, n0 + (int)rank * (OUT_COLS / 2), e_b);
+            tma_load_3d_pair(sb + C::B_BYTES / 2, &tmB2.m[own], lead_full, kb * BK, n0 + (int)rank * (OUT_COLS / 2), e_b);
           } else {
-            tma_load_3d_pair(sb, &tmB, lead_full, kb * BK, n0 + (int)rank * (BN / 2), t.e);
+            tma_load_3d_pair(sb, &tmB.m[own], lead_full, kb * BK, n0 + (int)rank * (BN / 2), e_b);
           }
         }
         __syncwarp();
@@ -1390,6 +1401,15 @@ static int make_tmap(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d1,
   return MOE_OK;
 }
 
+// maps of a weight of `groups` groups; the last of them at `last` where that is given
+static int make_weight_map(WeightMap* w, const void* base, const void* last, uint64_t K, uint64_t N, uint64_t groups, uint32_t box,
+                           int f16) {
+  int rc = make_tmap(&w->m[0], base, K, N, last ? groups - 1 : groups, box, f16);
+  if (rc) return rc;
+  w->m[1] = w->m[0];
+  return last ? make_tmap(&w->m[1], last, K, N, 1, box, f16) : MOE_OK;
+}
+
 // cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device attribute of a kernel: one flag per (kernel, device)
 template <class Kernel>
 static int allow_dynamic_smem(Kernel kernel, int bytes, std::atomic<bool>* done_per_device) {
@@ -1404,7 +1424,7 @@ static int allow_dynamic_smem(Kernel kernel, int bytes, std::atomic<bool>* done_
 }
 
 template <int MT, int BN, int EPI, bool GATHER, int AR = BM>
-static int launch_g(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2, const Params& p, int grid,
+static int launch_g(const CUtensorMap& tA, const WeightMap& tB, const WeightMap& tB2, const Params& p, int grid,
                     cudaStream_t st) {
   using C = Cfg<MT, BN, AR>;
   constexpr int SMEM = EPI == MOE_GEMM_PLAIN_F32 || EPI == MOE_GEMM_SILU_GATE ? C::SMEM_BYTES : C::SMEM_BYTES_STAGED;
@@ -1416,7 +1436,7 @@ static int launch_g(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensor
   return MOE_OK;
 }
 template <int MT, int BN, int EPI>
-static int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2, const Params& p, int grid,
+static int launch(const CUtensorMap& tA, const WeightMap& tB, const WeightMap& tB2, const Params& p, int grid,
                   cudaStream_t st) {
   // the row gather is compiled for the matrix epilogues only (the fused router has none)
   if (EPI != EPI_ROUTER && p.a_gather) return launch_g<MT, BN, EPI == EPI_ROUTER ? MOE_GEMM_PLAIN : EPI, true>(tA, tB, tB2, p, grid, st);
@@ -1424,7 +1444,7 @@ static int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMa
 }
 
 template <int EPI>
-static int launch_pair(const CUtensorMap& tA, const CUtensorMap& tA64, const CUtensorMap& tB, const CUtensorMap& tB2,
+static int launch_pair(const CUtensorMap& tA, const CUtensorMap& tA64, const WeightMap& tB, const WeightMap& tB2,
                        const Params& p, int grid, cudaStream_t st) {
   constexpr int SMEM = EPI == EPI_PEER || EPI == EPI_ROUTER ? PairCfg::SMEM_BYTES_STAGED : PairCfg::SMEM_BYTES;
   static std::atomic<bool> attr_set[64];
@@ -1446,6 +1466,8 @@ struct GatherArgs {           // A rows fetched through an index list instead of
   int w_slots = 0;            // see Params::w_slots
   bool pdl = false;           // behind another kernel of the same library call
   int64_t group_rows = 0;     // > 0: no group has more rows than this
+  const void* last_B = nullptr;    // weights of the last group where they do not lie behind the others' (with B2: both)
+  const void* last_B2 = nullptr;
 };
 
 static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const void* B2, const int32_t* offsets,
@@ -1473,13 +1495,15 @@ extern "C" int moe_grouped_gemm(int epilogue, const void* A, const void* B, cons
 int moe::grouped_gemm_gathered_ex(int epilogue, const void* X, int64_t x_rows, const int32_t* gather_idx, int gather_div,
                                   const void* B, const void* B2, const int32_t* offsets, const int32_t* dst_rows,
                                   const float* row_w, void* Y, int64_t ldy, int64_t max_rows, int64_t expected_rows, int K,
-                                  int N, int E, int dtype, int32_t* status, void* stream, bool pdl, int64_t group_rows) {
+                                  int N, int E, int dtype, int32_t* status, void* stream, bool pdl, int64_t group_rows,
+                                  const void* last_B, const void* last_B2) {
   if (!gather_idx) return fail(MOE_ERR_ARG, "grouped_gemm_gathered: null index list");
   if (gather_div < 1 || x_rows < 1 || x_rows > 0x7FFFFFFFll)
     return fail(MOE_ERR_ARG, "grouped_gemm_gathered: bad gather_div=%d or x_rows=%lld", gather_div, (long long)x_rows);
   if (K % 64) return fail(MOE_ERR_UNSUPPORTED, "grouped_gemm_gathered: K=%d must be a multiple of 64", K);
   GatherArgs ga;
   ga.idx = gather_idx; ga.div = gather_div; ga.src_rows = x_rows; ga.pdl = pdl; ga.group_rows = group_rows;
+  ga.last_B = last_B; ga.last_B2 = last_B2;
   return grouped_gemm_impl(epilogue, X, B, B2, offsets, dst_rows, row_w, Y, ldy, max_rows, K, N, E, status, stream,
                            nullptr, nullptr, 0, expected_rows, dtype, ga);
 }
@@ -1522,7 +1546,8 @@ int moe::router_topk_gemm(const void* x, const void* Wr, int64_t T, int H, int E
   p.dense_rows = (int)T;
   p.r_scores = scores; p.r_idx64 = indices; p.r_idx32 = indices32; p.r_logits = logits_out;
   p.r_k = k; p.r_mode = mode;
-  CUtensorMap tA, tB;
+  CUtensorMap tA;
+  WeightMap tB;
   rc = make_tmap(&tA, x, (uint64_t)H, (uint64_t)T, 0, (uint32_t)BM, f16);
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -1533,13 +1558,13 @@ int moe::router_topk_gemm(const void* x, const void* Wr, int64_t T, int H, int E
     // Measured (us; 16384 tokens, H = 7168, E = 256, k = 8, mode A): single CTAs, a list fed with every logit 97; pairs and
     // parked logits 82, with predicated parking 69 (HBM 36; the tensor pipe of the 128 SMs that hold a tile 44).  What is
     // left beside the tensor pipe is the epilogue of the one tile per CTA, which nothing overlaps.
-    rc = make_tmap(&tB, Wr, (uint64_t)H, (uint64_t)E, 1, 128u, f16);
+    rc = make_weight_map(&tB, Wr, nullptr, (uint64_t)H, (uint64_t)E, 1, 128u, f16);
     if (rc) return rc;
     const int64_t units = (T + 2 * BM - 1) / (2 * BM);
     const int pgrid = (int)(2 * units < dev.sm_count ? 2 * units : dev.sm_count) & ~1;
     return launch_pair<EPI_ROUTER>(tA, tA, tB, tB, p, pgrid, st);
   }
-  rc = make_tmap(&tB, Wr, (uint64_t)H, (uint64_t)E, 1, (uint32_t)E, f16);    // only the E weight rows are fetched
+  rc = make_weight_map(&tB, Wr, nullptr, (uint64_t)H, (uint64_t)E, 1, (uint32_t)E, f16);    // only the E weight rows are fetched
   if (rc) return rc;
   p.b_tx_bytes = E * BK * 2;
   const int64_t tiles = (T + BM - 1) / BM;
@@ -1549,8 +1574,9 @@ int moe::router_topk_gemm(const void* x, const void* Wr, int64_t T, int H, int E
 
 int moe::grouped_gemm_scatter_slots(const void* A, const void* B, const int32_t* offsets, const int32_t* dst_rows,
                                     const float* row_w, int w_slots, void* Y, int64_t ldy, int64_t max_rows, int K, int N,
-                                    int E, int dtype, int32_t* status, void* stream, bool pdl) {
+                                    int E, int dtype, int32_t* status, void* stream, bool pdl, const void* last_B) {
   GatherArgs ga;
+  ga.last_B = last_B;
   ga.w_slots = w_slots;
   ga.pdl = pdl;
   return grouped_gemm_impl(MOE_GEMM_SCALE_SCATTER_DSTW, A, B, nullptr, offsets, dst_rows, row_w, Y, ldy, max_rows, K, N, E,
@@ -1589,10 +1615,11 @@ int moe::gemm_splitk_f32(const void* A, const void* B, int64_t T, int K, int N, 
   p.dense_rows = (int)T;
   p.Y = Y; p.ldy = (int64_t)S * N;
   p.b_tx_bytes = N * BK * 2;
-  CUtensorMap tA, tB;
+  CUtensorMap tA;
+  WeightMap tB;
   rc = make_tmap(&tA, A, (uint64_t)K, (uint64_t)T, 0, (uint32_t)BM, f16);
   if (rc) return rc;
-  rc = make_tmap(&tB, B, (uint64_t)K, (uint64_t)N, 1, (uint32_t)N, f16);
+  rc = make_weight_map(&tB, B, nullptr, (uint64_t)K, (uint64_t)N, 1, (uint32_t)N, f16);
   if (rc) return rc;
   const int64_t tiles = ((T + BM - 1) / BM) * S;
   const int grid = (int)(tiles < dev.sm_count ? tiles : dev.sm_count);
@@ -1641,8 +1668,10 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
   if (epilogue == MOE_GEMM_SILU_GATE && !B2) return fail(MOE_ERR_ARG, "grouped_gemm: SILU_GATE needs the up weight");
   if (epilogue == MOE_GEMM_SCALE_SCATTER && !row_w) return fail(MOE_ERR_ARG, "grouped_gemm: SCALE_SCATTER needs row weights");
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(B2) |
-       reinterpret_cast<uintptr_t>(Y)) & 15)
+       reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(ga.last_B) | reinterpret_cast<uintptr_t>(ga.last_B2)) & 15)
     return fail(MOE_ERR_ARG, "grouped_gemm: pointers must be 16-byte aligned");
+  if (ga.last_B && (E < 2 || (epilogue == MOE_GEMM_SILU_GATE && !ga.last_B2)))
+    return fail(MOE_ERR_ARG, "grouped_gemm: a last group of its own needs another group and both of its weights");
   const int out_elem = epilogue == MOE_GEMM_PLAIN_F32 ? 4 : 2;
   if (ldy < N || (ldy * out_elem) % 16) return fail(MOE_ERR_ARG, "grouped_gemm: ldy=%lld must be >= N and 16-byte aligned", (long long)ldy);
   DeviceInfo dev;
@@ -1689,6 +1718,7 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
   p.w_by_dst = w_by_dst;
   p.w_slots = ga.w_slots;
   p.pdl = ga.pdl;
+  if (ga.last_B) p.b_groups = E - 1;
   p.y_rows = max_rows;     // a scatter permutes the sorted rows: the output has as many rows as the sorted input
   p.dense_rows = (int)ga.dense_rows;
   p.a_gather = ga.idx; p.a_src = A; p.a_div = ga.div; p.a_src_rows = (int)ga.src_rows; p.a_rows = (int)max_rows;
@@ -1703,7 +1733,8 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
   p.l2_hints = env_hints;
   p.mixed = env_mixed && offsets != nullptr;
 
-  CUtensorMap tA, tA64, tB, tB2;
+  CUtensorMap tA, tA64;
+  WeightMap tB, tB2;
   // with a row gather A is the un-permuted matrix (src_rows rows) and its tensor maps are never used by the kernel
   const uint64_t a_map_rows = ga.idx ? (uint64_t)ga.src_rows : (uint64_t)max_rows;
   rc = make_tmap(&tA, A, (uint64_t)K, a_map_rows, 0, (uint32_t)BM, f16);
@@ -1714,11 +1745,11 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
     if (rc) return rc;
     // a CTA of the pair stages 128 of the 256 N rows: one box, or a 64-row gate box and a 64-row up box
     const uint32_t box = gate ? 64u : 128u;
-    rc = make_tmap(&tB, B, (uint64_t)K, (uint64_t)N, (uint64_t)E, box, f16);
+    rc = make_weight_map(&tB, B, ga.last_B, (uint64_t)K, (uint64_t)N, (uint64_t)E, box, f16);
     if (rc) return rc;
     tB2 = tB;
     if (gate) {
-      rc = make_tmap(&tB2, B2, (uint64_t)K, (uint64_t)N, (uint64_t)E, box, f16);
+      rc = make_weight_map(&tB2, B2, ga.last_B2, (uint64_t)K, (uint64_t)N, (uint64_t)E, box, f16);
       if (rc) return rc;
     }
     const int64_t units = m_tiles_256 * p.num_n_tiles;
@@ -1736,11 +1767,11 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
   // accumulator columns it feeds are never stored)
   if (!gate && N < out_cols) b_box_rows = (uint32_t)N;
   p.b_tx_bytes = (int)b_box_rows * BK * 2 * (gate ? 2 : 1);
-  rc = make_tmap(&tB, B, (uint64_t)K, (uint64_t)N, (uint64_t)E, b_box_rows, f16);
+  rc = make_weight_map(&tB, B, ga.last_B, (uint64_t)K, (uint64_t)N, (uint64_t)E, b_box_rows, f16);
   if (rc) return rc;
   tB2 = tB;
   if (gate) {
-    rc = make_tmap(&tB2, B2, (uint64_t)K, (uint64_t)N, (uint64_t)E, b_box_rows, f16);
+    rc = make_weight_map(&tB2, B2, ga.last_B2, (uint64_t)K, (uint64_t)N, (uint64_t)E, b_box_rows, f16);
     if (rc) return rc;
   }
   const int64_t tiles_bound = m_tiles_128 * p.num_n_tiles;

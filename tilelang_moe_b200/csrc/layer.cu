@@ -17,11 +17,13 @@ struct LayerScratch {
 };
 
 // The shared expert can ride along as expert E of the routed GEMMs - every token then has k + 1 routed entries, the
-// last with weight 1 - when it has the width of a routed expert and its weights lie directly behind the routed ones
-// in memory (one [E+1, ...] tensor per projection), and the up GEMM gathers its rows itself.
-static bool shared_rides_along(const void* shared_gate, const void* shared_up, const void* shared_down, const void* routed_gate,
-                               const void* routed_up, const void* routed_down, int H, int I, int E, int SI) {
-  if (SI != I || SI == 0 || H % 64 || E + 1 > 1024) return false;
+// last with weight 1 - when it has the width of a routed expert and the up GEMM gathers its rows itself.  The GEMMs read
+// its weights where they lie.
+static bool shared_can_ride(int H, int I, int E, int SI) { return SI == I && SI > 0 && H % 64 == 0 && E + 1 <= 1024; }
+
+// ... which a caller of moe_layer_forward asks for by keeping one [E+1, ...] tensor per projection
+static bool shared_lies_behind(const void* shared_gate, const void* shared_up, const void* shared_down, const void* routed_gate,
+                               const void* routed_up, const void* routed_down, int H, int I, int E) {
   const size_t per = (size_t)I * H * 2;
   return reinterpret_cast<const unsigned char*>(routed_gate) + (size_t)E * per == shared_gate &&
          reinterpret_cast<const unsigned char*>(routed_up) + (size_t)E * per == shared_up &&
@@ -135,9 +137,20 @@ extern "C" int moe_layer_forward(const void* x, const void* router_weight, const
                                  const void* routed_up, const void* routed_down, int64_t T, int H, int I, int E, int k,
                                  int SI, int dtype, void* ws, size_t ws_bytes, void* out, int32_t* status, void* stream,
                                  void* side_stream) {
+  return moe_layer_forward_ex(x, router_weight, logits, shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down, T,
+                              H, I, E, k, SI, dtype, ws, ws_bytes, out, status, stream, side_stream, 0);
+}
+
+extern "C" int moe_layer_forward_ex(const void* x, const void* router_weight, const float* logits, const void* shared_gate,
+                                    const void* shared_up, const void* shared_down, const void* routed_gate,
+                                    const void* routed_up, const void* routed_down, int64_t T, int H, int I, int E, int k,
+                                    int SI, int dtype, void* ws, size_t ws_bytes, void* out, int32_t* status, void* stream,
+                                    void* side_stream, int shared_group) {
   using namespace moe;
   if (T < 0 || H < 8 || (H % 8) || I < 8 || (I % 8) || E < 1 || k < 1 || k > E || SI < 0 || (SI % 8))
     return fail(MOE_ERR_ARG, "layer_forward: bad shape T=%lld H=%d I=%d E=%d k=%d SI=%d", (long long)T, H, I, E, k, SI);
+  if (shared_group && !shared_can_ride(H, I, E, SI))
+    return fail(MOE_ERR_ARG, "layer_forward: a shared expert of %d columns cannot be a group of experts of %d (H=%d E=%d)", SI, I, H, E);
   if (T == 0) return MOE_OK;
   if (!x || (!router_weight && !logits) || !routed_gate || !routed_up || !routed_down || !out || !ws)
     return fail(MOE_ERR_ARG, "layer_forward: null pointer");
@@ -170,9 +183,10 @@ extern "C" int moe_layer_forward(const void* x, const void* router_weight, const
     return code;
   };
 
-  // shared expert: one more group of the routed GEMMs where its weights allow it; else it depends on x only and runs
+  // shared expert: one more group of the routed GEMMs where that is asked for; else it depends on x only and runs
   // beside the routed path when a second stream is given
-  const bool ride = SI > 0 && shared_rides_along(shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down, H, I, E, SI);
+  const bool ride = shared_group || (shared_can_ride(H, I, E, SI) && shared_lies_behind(shared_gate, shared_up, shared_down,
+                                                                                        routed_gate, routed_up, routed_down, H, I, E));
   void* shared_out = nullptr;
   if (SI > 0 && !ride) {
     void* sst = stream;
@@ -227,9 +241,10 @@ routed:
                             moe_route_histogram_workspace(n1, E + 1), status, stream, k, pdl);
     if (rc) return rc;
     rc = grouped_gemm_gathered_ex(MOE_GEMM_SILU_GATE, x, T, perm, k + 1, routed_gate, routed_up, offsets, nullptr, nullptr, act,
-                                   I, n1, 0, H, I, E + 1, dtype, status, stream, pdl, T);
+                                   I, n1, 0, H, I, E + 1, dtype, status, stream, pdl, T, shared_gate, shared_up);
     if (rc) return rc;
-    rc = grouped_gemm_scatter_slots(act, routed_down, offsets, perm, scores, k, yk, H, n1, I, H, E + 1, dtype, status, stream, pdl);
+    rc = grouped_gemm_scatter_slots(act, routed_down, offsets, perm, scores, k, yk, H, n1, I, H, E + 1, dtype, status, stream, pdl,
+                                    shared_down);
     if (rc) return rc;
     return combine_ex(yk, nullptr, nullptr, nullptr, T, k + 1, H, dtype, out, stream, pdl);
   }

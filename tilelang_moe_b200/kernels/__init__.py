@@ -89,6 +89,27 @@ def grouped_gemm(X: torch.Tensor, W: torch.Tensor, expert_indices: torch.Tensor,
 grouped_gemm_best = grouped_gemm
 
 
+def _stackable(weights, E: int, I: int, H: int):
+    """The six expert weights (shared gate, up, down; routed ones) as the GEMMs read them: where they are, or copies of
+    those that have another shape, type or device, are not contiguous or do not start on a 16-byte boundary."""
+    sg, su, sd, rg, ru, rd = weights
+    up, down, n = (I, H), (H, I), I * H
+    if (sg.shape == up and su.numel() == n and sd.numel() == n and ru.shape == rg.shape and rd.shape == (E, H, I)
+            and not (sg.data_ptr() | su.data_ptr() | sd.data_ptr() | rg.data_ptr() | ru.data_ptr() | rd.data_ptr()) & 15
+            and sg.is_contiguous() and su.is_contiguous() and sd.is_contiguous()
+            and rg.is_contiguous() and ru.is_contiguous() and rd.is_contiguous()
+            and sg.dtype is su.dtype is sd.dtype is rg.dtype is ru.dtype is rd.dtype
+            and sg.get_device() == su.get_device() == sd.get_device() == rg.get_device()):
+        return weights
+
+    def laid_out(w):
+        return w if w.is_contiguous() and not w.data_ptr() & 15 else w.clone(memory_format=torch.contiguous_format)
+
+    routed = [w.expand(E, *shape) for w, shape in ((rg, up), (ru, up), (rd, down))]
+    shared = [w.reshape(shape).to(r) for w, r, shape in ((sg, rg, up), (su, ru, up), (sd, rd, down))]
+    return [laid_out(w) for w in (*shared, *routed)]
+
+
 class FusedMoETileLang:
     """Shared + routed SiLU-gated MoE layer with persistent scratch for one shape.
 
@@ -110,38 +131,27 @@ class FusedMoETileLang:
                                              n_routed_experts, d_expert * n_shared_experts, dev, dtype)
 
     # A single shared expert of the routed experts' width can run as expert E of the routed grouped GEMMs (five
-    # launches for the whole layer, no second stream): the library does so when the shared weights lie directly behind
-    # the routed ones in memory.  The layer object keeps such stacked copies of the weights it is called with, as the
-    # reference's layer keeps its stacked expert tensors (kernels/fusedmoe_tilelang.py:296-307), as long as they stay
-    # below this size; larger layers keep the side-stream form and their weights where they are.
+    # launches for the whole layer, no second stream).  The GEMMs read every weight where the caller keeps it: the layer
+    # object holds no copy that a later write to a weight, by whatever means, could leave behind.  Layers whose weights
+    # exceed this size keep the side-stream form.
     STACK_LIMIT_BYTES = 2 << 30
+    _stack = None       # (E + 1, I, H) of the experts that the last forward ran as one stack, None for the side-stream form
 
-    def _stacked(self, shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down):
-        ws = (shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down)
+    def _stack_shape(self, shared_gate, shared_up, shared_down, routed_gate):
         E, I, H = routed_gate.shape
-        if (self.n_shared_experts != 1 or H % 64 or any(w is None for w in ws)
+        if (self.n_shared_experts != 1 or H % 64 or E >= 1024 or shared_gate is None or shared_up is None or shared_down is None
                 or 3 * (E + 1) * I * H * routed_gate.element_size() > self.STACK_LIMIT_BYTES):
             return None
-        key = tuple((w.data_ptr(), w._version) for w in ws)
-        if getattr(self, "_stack_key", None) != key:
-            def stack(routed, shared, shape):
-                out = torch.empty(E + 1, *shape, dtype=routed.dtype, device=routed.device)
-                out[:E].copy_(routed)
-                out[E].copy_(shared.reshape(shape))
-                return out
-            g, u, d = (stack(routed_gate, shared_gate, (I, H)), stack(routed_up, shared_up, (I, H)),
-                       stack(routed_down, shared_down, (H, I)))
-            self._stack = (g[E], u[E], d[E], g[:E], u[:E], d[:E])       # the views every forward passes on
-            self._stack_key = key
-        return self._stack
+        return E + 1, I, H
 
     def forward(self, x, router_weight, shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down,
                 logits: Optional[torch.Tensor] = None):
         """One library call (``moe_layer_forward``) enqueues the whole layer."""
-        st = self._stacked(shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down) \
-            if self.n_shared_experts else None
+        st = self._stack = self._stack_shape(shared_gate, shared_up, shared_down, routed_gate)
         if st is not None:
-            return _layer.moe_forward_single_call(x, router_weight, *st, self.n_experts_per_token, ws=self.ws, logits=logits)
+            weights = _stackable((shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down), st[0] - 1, st[1], st[2])
+            return _layer.moe_forward_single_call(x, router_weight, *weights, self.n_experts_per_token, ws=self.ws, logits=logits,
+                                                  shared_group=True)
         return _layer.moe_forward_single_call(x, router_weight, shared_gate if self.n_shared_experts else None,
                                               shared_up, shared_down, routed_gate, routed_up, routed_down,
                                               self.n_experts_per_token, ws=self.ws, logits=logits)

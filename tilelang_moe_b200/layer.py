@@ -187,9 +187,10 @@ class SingleCallWorkspace:
 def moe_forward_single_call(x: torch.Tensor, router_weight: Optional[torch.Tensor], shared_gate, shared_up, shared_down,
                             routed_gate: torch.Tensor, routed_up: torch.Tensor, routed_down: torch.Tensor, k: int,
                             ws: Optional[SingleCallWorkspace] = None, logits: Optional[torch.Tensor] = None,
-                            out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                            out: Optional[torch.Tensor] = None, shared_group: bool = False) -> torch.Tensor:
     """The layer through ``moe_layer_forward``: one library call enqueues every kernel (the shared expert on the
-    side stream), instead of one Python-level call per stage.  Same kernels, same results as ``moe_forward``."""
+    side stream, or with ``shared_group`` as one more group of the routed GEMMs), instead of one Python-level call per
+    stage.  Same kernels, same results as ``moe_forward``."""
     if x.dtype not in ops.DTYPE_CODE:
         raise ValueError("moe_b200 computes in bfloat16 or float16; cast the activations and weights")
     shape = x.shape
@@ -213,14 +214,14 @@ def moe_forward_single_call(x: torch.Tensor, router_weight: Optional[torch.Tenso
     if ws is None or ws.key != key:
         ws = SingleCallWorkspace(T, k, H, I, E, SI, dev, x.dtype)
     y = ws.out if out is None else out.view(T, H)
-    side = _side_stream(dev) if SI > 0 else None
+    side = _side_stream(dev) if SI > 0 and not shared_group else None
     p = ops._ptr
     with ops._on(dev):
-        rc = _lib.load().moe_layer_forward(
+        rc = _lib.load().moe_layer_forward_ex(
             p(x_flat), p(router_weight) if logits is None else None, p(logits), p(shared_gate), p(shared_up), p(shared_down),
             p(routed_gate), p(routed_up), p(routed_down), T, H, I, E, k, SI, ops.DTYPE_CODE[x.dtype],
             ws.buf.data_ptr() + ws.offset, ws.bytes, p(y), p(ops.status_buffer(dev)), ops._stream(),
-            side.cuda_stream if side is not None else None)
+            side.cuda_stream if side is not None else None, int(shared_group))
     _lib.check(rc, "moe_layer_forward")
     ops._after(dev)
     return y.view(*shape)
