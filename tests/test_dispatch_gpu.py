@@ -115,3 +115,35 @@ def test_up_gemm_of_few_rows(cuda, lib, T, H, I, E, k, shared, dtype):
     plain = ops.grouped_gemm_sorted(ops.GEMM_SILU_GATE, xs[perm.long()].to(cuda), ws[4], offs.to(cuda), B2=ws[5])
     ops.check_status(cuda)
     assert torch.equal(act, plain)
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 256, 8), (33, 256, 8), (257, 136, 7), (130, 64, 8), (31, 40, 8), (1000, 128, 3)])
+@pytest.mark.parametrize("kind", ["nan", "inf", "zero rows"])
+def test_router_selection_of_special_logits(cuda, lib, T, E, k, kind):
+    """One-kernel router on ragged batches with NaN and infinite logits and with rows of zeros (padding tokens).  Each expert's
+    weight picks columns of x, so the logits are known exactly."""
+    H = 64
+    g = torch.Generator().manual_seed(T + E + k)
+    X = (torch.round(torch.randn(T, H, generator=g) * 4) / 4).bfloat16()
+    W = torch.zeros(E, H)
+    W[torch.arange(E), torch.arange(E) % 60] = 1.0 + torch.arange(E) // 60 * 0.25
+    special = torch.rand(T, generator=g) < 0.4
+    if kind == "nan":                             # NaN times zero: the whole row
+        X[special, 3] = float("nan")
+    elif kind == "inf":
+        X[:, 62] = 0.0
+        X[special, 62] = float("inf")
+        W[:, 62] = torch.where(torch.arange(E) % 3 == 1, 1.0, -1.0)
+    else:
+        X[special] = 0.0
+    X, W = X.to(cuda), W.bfloat16().to(cuda)
+    lg = torch.full((T, E), float("nan"), device=cuda)
+    for mode in ("B", "A"):
+        s, i = ops.router_topk_softmax(X, W, k, mode=mode, logits_out=lg, fused=True)
+        ops.check_status(cuda)
+        torch.testing.assert_close(lg, ops.router_logits(X, W), rtol=0, atol=0, equal_nan=True)
+        s_ref, i_ref = O.topk_softmax(lg.cpu(), k, mode)
+        assert torch.equal(i.cpu(), i_ref)
+        ok = lg.cpu().isfinite().all(1)
+        torch.testing.assert_close(s.cpu()[ok], s_ref[ok], rtol=1e-6, atol=1e-30)
+        assert kind == "inf" or s.cpu()[~ok].isnan().all()
