@@ -449,8 +449,14 @@ __device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(
 // it: about 11 thousand instructions per tile, and with one tile per CTA nothing hides them.  Instead the first pass
 // keeps only the eight largest of the maxima of eight neighbouring columns; the k-th of them, V, is a lower bound of the
 // k-th largest logit.  The second pass parks the logits not below V in shared memory (NaNs are not; they do not enter V
-// either) and adds up the softmax denominator; those, a dozen as a rule, go through the list in column order.  A warp
-// with more than ROUTER_CAP of them in one row feeds the list from tensor memory after all.
+// either) and adds up the softmax denominator; those, a dozen as a rule, go through the list in column order.  Where a row
+// has more than ROUTER_CAP of them (few experts, equal logits, ascending ones), the warp passes over tensor memory again
+// and parks what lies behind them and above the list's k-th entry so far, until nothing is left.  At most 64 logits of a
+// row differ and lie above V (eight groups of eight), equal ones drop out with the first k, so a few passes do.
+// Measured (us, 16384 tokens, k = 8; a list fed with every logit, in all rows -> in warps with such a row -> further passes):
+// H = 7168, E = 64 52.8 -> 52.0 -> 49.5, E = 136 69.2 -> 62.0 -> 54.6, E = 256 with a twentieth of the rows zero
+// 85.8 -> 74.0 -> 61.2; H = 1024, E = 96 22.5 -> 21.8 -> 16.7.  The one loss: logits that ascend with the expert in every
+// row, E = 64 52.7 -> 51.8 -> 53.3.
 constexpr int ROUTER_CAP = 16;
 static_assert((ROUTER_CAP + 1) * 256 <= 32 * Cfg<1, 128>::STAGING_PITCH, "parked logits of a warp fit its staging rows");
 __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t taddr, int grow, bool row_ok,
@@ -540,23 +546,45 @@ __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t ta
   int kv[KMAX], ki[KMAX];
 #pragma unroll
   for (int j = 0; j < KMAX; ++j) { kv[j] = (int)0x80000000; ki[j] = 0; }
-  if (!__any_sync(0xFFFFFFFFu, cnt > ROUTER_CAP)) {
-    for (int j = 0; j < cnt; ++j) {         // ascending columns and a strict comparison: lowest index first among equals
-      const float2 e = mine[32 * j];
+  for (;;) {
+    const bool more = cnt > ROUTER_CAP;
+    for (int j = 0; j < (more ? ROUTER_CAP : cnt); ++j) {   // ascending columns and a strict comparison: lowest index first
+      const float2 e = mine[32 * j];                        // among equals
       list_insert<KMAX>(kv, ki, float_to_ikey(e.x), __float_as_int(e.y));
     }
-    __syncwarp();                           // tensor-memory loads below and in the next tile are warp-wide
-  } else {
+    if (!__any_sync(0xFFFFFFFFu, more)) break;              // also: tensor-memory loads are warp-wide
+    // Some row had more entries than it may park.  What can still enter its list lies behind the last one parked and above
+    // the list's k-th: an equal logit loses to the earlier column, and nothing is above a NaN.
+    int kth = kv[0];
+#pragma unroll
+    for (int j = 1; j < KMAX; ++j) kth = j < p.r_k ? kv[j] : kth;
+    const float bound = ikey_to_float(kth);
+    const int behind = more && bound == bound ? __float_as_int(mine[32 * (ROUTER_CAP - 1)].y) : 0x7FFFFFFF;
+    at = first;
+    cnt = 0;
 #pragma unroll 1
     for (int c = 0; c < chunks; ++c) {
       uint32_t v[32];
       tmem_ld32(taddr + c * 32, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int col = c * 32 + j;
-        const int key = float_to_ikey(__uint_as_float(v[j]));
-        if (col < p.N && key > kv[KMAX - 1]) list_insert<KMAX>(kv, ki, key, col);
+      for (int q = 0; q < 4; ++q) {
+        if (c * 32 + q * 8 < p.N) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.gtu.f32 p, %2, %3;\n\t"               // above the bound: also true for NaN
+                "setp.gt.and.s32 p, %5, %7, p;\n\t"
+                "@p st.shared.v2.b32 [%0], {%4, %5};\n\t"
+                "@p add.s32 %1, %1, 1;\n\t"
+                "@p add.u32 %0, %0, 256;\n\t"
+                "min.u32 %0, %0, %6;\n\t}"
+                : "+r"(at), "+r"(cnt)
+                : "f"(__uint_as_float(v[8 * q + j])), "f"(bound), "r"(v[8 * q + j]), "r"(c * 32 + q * 8 + j), "r"(last), "r"(behind)
+                : "memory");
+          }
+        }
       }
     }
   }
