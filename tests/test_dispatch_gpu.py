@@ -147,3 +147,31 @@ def test_router_selection_of_special_logits(cuda, lib, T, E, k, kind):
         ok = lg.cpu().isfinite().all(1)
         torch.testing.assert_close(s.cpu()[ok], s_ref[ok], rtol=1e-6, atol=1e-30)
         assert kind == "inf" or s.cpu()[~ok].isnan().all()
+
+
+@pytest.mark.parametrize("form", ["128", "pair", "few rows"])
+def test_silu_over_its_whole_range(cuda, lib, monkeypatch, form):
+    """SiLU epilogue on gates up to where exp(-g) overflows (g = -88.7; its denominator passes 2^126 at -87.3), past that, on
+    infinities and NaN.  A gate is a sum of two weights, so it is exact; exp is within 2^-17, the result rounded to bf16 once."""
+    if form != "few rows":
+        monkeypatch.setenv("MOE_B200_GEMM_TILE_ROWS", form)
+    g = torch.cat([torch.arange(-5673, -5586) / 64, torch.linspace(-87, 20, 400), torch.tensor([0.0, 1e-20, -1e-20, 300.0, 1e30]),
+                   torch.tensor([-89.0, -200.0, -1e30, float("inf"), float("-inf"), float("nan")])])
+    g = torch.cat([g, torch.zeros(-len(g) % 64)])
+    N, K, rows = len(g), 64, 5 if form == "few rows" else 300
+    hi = g.bfloat16()
+    lo = torch.where(hi.isfinite(), g - hi.float(), 0.0).bfloat16()
+    gate = hi.double() + lo.double()
+    Wg, Wu, A = torch.zeros(1, N, K), torch.zeros(1, N, K), torch.zeros(rows, K)
+    Wg[0, :, 0], Wg[0, :, 1], Wu[0, :, 0], A[:, 0], A[:, 1] = hi.float(), lo.float(), 1.0, 1.0, 1.0
+    args = [t.bfloat16().to(cuda) for t in (A, Wg, Wu)]
+    offs = torch.tensor([0, rows], dtype=torch.int32, device=cuda)
+    gather = torch.arange(rows, dtype=torch.int32, device=cuda) if form == "few rows" else None
+    y = ops.grouped_gemm_sorted(ops.GEMM_SILU_GATE, args[0], args[1], offs, B2=args[2], gather=gather).cpu().double()
+    ops.check_status(cuda)
+    exact = gate / (1.0 + torch.exp(-gate))
+    near = gate.isfinite() & (gate >= -88.65)
+    torch.testing.assert_close(y[:, near], exact[near].expand(rows, -1), rtol=2.0 ** -8, atol=0)
+    far = gate.isfinite() & (gate < -88.65)
+    assert far.any() and bool(((y[:, far] <= 0) & (y[:, far] > -1e-35)).all())
+    assert bool((y[:, gate == float("inf")] == float("inf")).all()) and bool(y[:, ~gate.isfinite() & (gate != float("inf"))].isnan().all())
