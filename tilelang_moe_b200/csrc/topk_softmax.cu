@@ -568,7 +568,8 @@ constexpr int RT = 512;             // threads per CTA
 constexpr int RWARPS = RT / 32;
 constexpr int RBINS = 2048;         // histogram bins (11-bit digit)
 constexpr int RBPT = RBINS / RT;    // bins owned by one thread in the scan (4)
-constexpr int RCTRL_BYTES = 256;
+constexpr int RCTRL_BYTES = 288;
+constexpr int RCHUNKS = 512;        // 128-byte chunks of a row that one CTA holds (RMAX_SLICE / 32; one per thread in their scan)
 constexpr int RMAX_SLICE = 16384;   // keys one CTA holds (32 per thread)
 constexpr int RMAX_KPAD = 4096;
 
@@ -582,8 +583,10 @@ struct RadixCtrl {
   uint32_t loc_count;   // collected entries of this CTA
   double blk_sum;       // this CTA's share of the full-row denominator (modes A)
   double sel_sum;       // ... of a sum over the k selected
+  uint2 cand[3];        // this CTA's candidates in passes 1, 2 and 3: smallest key, complement of the largest
 };
-static_assert(sizeof(RadixCtrl) <= RCTRL_BYTES, "control block too large");
+static_assert(sizeof(RadixCtrl) <= RCTRL_BYTES && RCTRL_BYTES % 16 == 0, "control block too large");
+static_assert(RMAX_SLICE / 32 <= RCHUNKS && RCHUNKS <= RT, "a thread per chunk");
 
 __device__ __forceinline__ uint64_t pack_entry(uint32_t key, uint32_t col) {
   return ((uint64_t)key << 32) | (uint64_t)(0xFFFFFFFFu - col);
@@ -676,17 +679,20 @@ __device__ __forceinline__ uint32_t count_above(const uint64_t* a, uint32_t n, u
 
 // One cluster of C CTAs per row.  The row's 128-byte chunks go round the CTAs (a row in sorted order is spread evenly), each
 // keeps its share as keys in registers, KPT per thread.
-//   1. radix select on key | column, 11 / 11 / 10 bits of the key, then 11 / 6 of the column among equal keys: histograms of
-//      all CTAs are added over distributed shared memory.  It stops as soon as the entries not below the selected bin are
-//      few enough to be sorted outright (totcap), after one digit as a rule.
+//   1. radix select on the key, 11 / 11 / 10 bits: histograms of all CTAs are added over distributed shared memory.  It stops
+//      as soon as the entries not below the selected bin are few enough to be sorted outright (totcap), after one digit as a
+//      rule.  Where the bin holds one value only (masked, constant or quantised rows; after three digits in any case), as many
+//      of its entries as are needed are taken in column order: the CTAs exchange their counts per chunk at the same barrier.
 //   2. every CTA collects those of its share and sorts them;
 //   3. it copies the other CTAs' sorted entries; an entry's place in the row's order is its place in its own list plus, by
 //      binary search, the entries of the other lists ahead of it.  Places below k are written out.
 // What bounds it: latency (barriers, shared-memory atomics, the sort's chain of exchanges).
 // Measured (us, gathering the k selected into the leading CTA and sorting them there after all three digits -> this):
-// 64 x 32768, k = 2048: 44.0 -> 31.4; one such row 30.4 -> 19.6; 4096 x 4096, k = 64: 177 -> 140; 256 x 32768, k = 2048:
-// 100 -> 93; 16 x 65536, k = 1024: 34.9 -> 26.1; 64 x 32768, k = 32: 19.8 -> 16.8.  Rows of equal logits alone pay for the
-// two more digits: 64 x 32768, k = 32 20.2 -> 27.1, k = 2048 45.5 -> 33.5.
+// 64 x 32768, k = 2048: 43.7 -> 30.9; one such row 30.6 -> 19.3; 4096 x 4096, k = 64: 178 -> 138; 256 x 32768, k = 2048: 99.8 -> 88.5;
+// 16 x 65536, k = 1024: 34.7 -> 26.4; 64 x 32768, k = 32: 19.8 -> 17.1.  Rows of equal logits (with two more digits, of the
+// column, in place of the counts per chunk: in brackets): 64 x 32768, k = 32 20.2 -> 21.3 [26.8], k = 2048 45.4 -> 28.0 [32.9];
+// 4096 x 2048, k = 8 138 -> 132 [201].  The counts cost registers: rows above 65536 that need all three digits and hold no
+// ties, 32 x 131072, k = 64 35.8 -> 39.5 [35.7].
 template <int KPT>
 __global__ void __launch_bounds__(RT, 2)
 topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld, int k, int totcap, int lcap, int mode,
@@ -702,11 +708,14 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
 
   RadixCtrl* ctrl = reinterpret_cast<RadixCtrl*>(smem_raw);
   uint32_t* hist = reinterpret_cast<uint32_t*>(smem_raw + RCTRL_BYTES);
-  uint64_t* lbuf = reinterpret_cast<uint64_t*>(smem_raw + RCTRL_BYTES + 2 * RBINS * 4);   // [lcap] this CTA's entries
+  uint32_t* chunk_n = hist + 2 * RBINS;      // candidates per chunk of this CTA, read by the others
+  uint32_t* chunk_at = chunk_n + RCHUNKS;    // candidates of the row in the chunks before each of them
+  uint64_t* lbuf = reinterpret_cast<uint64_t*>(chunk_at + RCHUNKS);                       // [lcap] this CTA's entries
   uint64_t* others = lbuf + lcap;                                                         // [totcap] the other CTAs'
 
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (tid == 0) { ctrl->blk_maxkey = 0u; ctrl->blk_sum = 0.0; ctrl->sel_bin = 0u; ctrl->k_rem = 0u; ctrl->bin_count = 0u; }
+  if (tid < 3) ctrl->cand[tid] = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
   for (int i = tid; i < 2 * RBINS; i += RT) hist[i] = 0u;
 
   // ---- this CTA's share as keys (the only read of the logits); 0 where there is none (no float has that key)
@@ -741,33 +750,60 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
     if (lane == 0) atomicMax(&ctrl->blk_maxkey, lmax);
   }
 
-  // ---- 1. radix select: `prefix` is the lowest key of the bin that holds the k-th largest entry (after three digits its key),
-  //      `cprefix` the same of CMAX - column among equal keys
-  constexpr int CMAX = (1 << 17) - 1;                 // N <= 8 * RMAX_SLICE = 2^17
-  uint32_t prefix = 0u, pmask = 0u, cprefix = 0u, cmask = 0u, k_rem = (uint32_t)k;
+  // ---- 1. radix select: `prefix` is the lowest key of the bin that holds the k-th largest entry (after three digits its key)
+  uint32_t prefix = 0u, pmask = 0u, k_rem = (uint32_t)k;
+  uint32_t m = 0u;                                    // keys that are taken
   double rowsum = 0.0;
+  bool tied = false;
+  auto count = [&](int w, uint32_t value) {         // this thread's keys of that value in vectors 4w .. 4w + 3, a byte each
+    uint32_t n = 0u;
+#pragma unroll
+    for (int j = 16 * w; j < 16 * w + 16 && j < KPT; ++j) n += key[j] == value ? 1u << (8 * ((j >> 2) & 3)) : 0u;
+    return n;
+  };
 #pragma unroll 1
-  for (int pass = 0; pass < 5; ++pass) {
-    const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : (pass == 3 ? 6 : 0));
-    const uint32_t dmask = pass == 2 ? 1023u : (pass == 4 ? 63u : 2047u);
+  for (int pass = 0; pass < 4; ++pass) {
+    const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
+    const uint32_t dmask = pass == 2 ? 1023u : 2047u;
     uint32_t* h = hist + (pass & 1) * RBINS;
-    if (pass >= 2) {  // this buffer again: every remote read of it ended before the last pass's cluster barrier
+    if (pass == 2) {  // this buffer again: every remote read of it ended before the last pass's cluster barrier
       for (int i = tid; i < RBINS; i += RT) h[i] = 0u;
       __syncthreads();
     }
-    if (pass < 3) {
+    uint32_t lo = 0xFFFFFFFFu, hi = 0u;               // smallest and largest candidate of this warp, then of the row
+    if (pass == 0) {
 #pragma unroll
       for (int j = 0; j < KPT; ++j)
-        if (key[j] != 0u && (key[j] & pmask) == prefix) atomicAdd(&h[(key[j] >> shift) & dmask], 1u);
+        if (key[j] != 0u) atomicAdd(&h[key[j] >> 21], 1u);
     } else {
 #pragma unroll
       for (int j = 0; j < KPT; ++j) {
-        const uint32_t inv = (uint32_t)(CMAX - col_of(j));
-        if (key[j] == prefix && (inv & cmask) == cprefix) atomicAdd(&h[(inv >> shift) & dmask], 1u);
+        if (key[j] != 0u && (key[j] & pmask) == prefix) {
+          if (pass < 3) atomicAdd(&h[(key[j] >> shift) & dmask], 1u);
+          lo = min(lo, key[j]);
+          hi = max(hi, key[j]);
+        }
+      }
+    }
+    if (pass > 0) {
+      lo = __reduce_min_sync(FULL, lo);
+      hi = __reduce_max_sync(FULL, hi);
+      if (lane == 0 && hi != 0u) { atomicMin(&ctrl->cand[pass - 1].x, lo); atomicMin(&ctrl->cand[pass - 1].y, ~hi); }
+      if (lo >= hi) {                                 // one value, or none: else the counts are of no use
+#pragma unroll
+        for (int w = 0; w < (KPT + 15) / 16; ++w) {   // over the eight lanes of a chunk
+          uint32_t v = hi != 0u ? count(w, lo) : 0u;
+#pragma unroll
+          for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+          if ((lane & 7) < 4 && 4 * w + (lane & 7) < KPT / 4)
+            chunk_n[(4 * w + (lane & 7)) * (RT / 8) + (tid >> 3)] = (v >> (8 * (lane & 7))) & 0xFFu;
+        }
       }
     }
     cluster.sync();
 
+    uint2 cand = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+    if (pass > 0 && (unsigned)lane < C) cand = cluster.map_shared_rank(ctrl, lane)->cand[pass - 1];
     uint32_t g[RBPT];
 #pragma unroll
     for (int j = 0; j < RBPT; ++j) g[j] = 0u;
@@ -778,6 +814,11 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
         const uint4 v = *reinterpret_cast<const uint4*>(rh + tid * RBPT);
         g[0] += v.x; g[1] += v.y; g[2] += v.z; g[3] += v.w;
       }
+    }
+    if (pass > 0) {
+      lo = __reduce_min_sync(FULL, cand.x);
+      hi = ~__reduce_min_sync(FULL, cand.y);
+      if (lo == hi) { prefix = lo; tied = true; break; }   // the same in every CTA of the cluster
     }
     const uint32_t tsum = g[0] + g[1] + g[2] + g[3];
     uint32_t inc = tsum;  // suffix-inclusive sum over lanes >= lane
@@ -803,8 +844,8 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
     const uint32_t bin = ctrl->sel_bin;
     k_rem = ctrl->k_rem;
     const uint32_t total_ge = (uint32_t)k - k_rem + ctrl->bin_count;
-    if (pass < 3) { prefix |= bin << shift; pmask |= dmask << shift; }
-    else { cprefix |= bin << shift; cmask |= dmask << shift; }
+    prefix |= bin << shift;
+    pmask |= dmask << shift;
 
     if (pass == 0 && mode != MOE_TOPK_MODE_B) {
       // full-row softmax denominator: cluster max, then this CTA's share of sum exp(v - max)
@@ -818,17 +859,59 @@ topk_radix_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
       part = block_sum_ordered(part, ctrl, lane, wid);
       if (tid == 0) ctrl->blk_sum = part;  // published by the next cluster barrier
     }
-    if (total_ge <= (uint32_t)totcap) break;          // the same in every CTA of the cluster; all five digits leave k entries
+    if (total_ge <= (uint32_t)totcap) break;          // the same in every CTA of the cluster; pass 3 never gets here
     __syncthreads();                                  // every thread has read the selection before the next pass replaces it
   }
 
-  // ---- 2. collect
-  uint32_t m = 0u;
+  if (tied) {                                         // k_rem of the entries equal to prefix
+    // thread t: chunk t of every CTA.  Row order is chunk by chunk, and within a chunk number the CTAs in turn
+    uint32_t all = 0u, ahead = 0u;
+    if (tid < KPT * 16) {
 #pragma unroll
-  for (int j = 0; j < KPT; ++j) {
-    const bool in = key[j] > prefix || (key[j] == prefix && (uint32_t)(CMAX - col_of(j)) >= cprefix);
-    m |= (key[j] != 0u && in) ? (1u << j) : 0u;
+      for (unsigned c = 0; c < 8; ++c) {
+        if (c < C) {
+          const uint32_t v = cluster.map_shared_rank(chunk_n, c)[tid];
+          all += v;
+          if (c < crank) ahead += v;
+        }
+      }
+    }
+    uint32_t inc = all;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, inc, o);
+      if (lane >= o) inc += v;
+    }
+    if (lane == 31) ctrl->warp_tot[wid] = inc;
+    __syncthreads();
+    uint32_t before = ahead + inc - all;
+#pragma unroll
+    for (int w = 0; w < RWARPS; ++w) before += w < wid ? ctrl->warp_tot[w] : 0u;
+    chunk_at[tid] = before;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < (KPT + 15) / 16; ++w) {
+      const uint32_t own = count(w, prefix);
+      uint32_t lower = own;                       // candidates of the chunk's lanes up to this one: at most 32, a byte each
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, lower, o, 8);
+        if ((lane & 7) >= o) lower += v;
+      }
+      lower -= own;
+#pragma unroll
+      for (int q = 4 * w; q < KPT / 4 && q < 4 * w + 4; ++q) {
+        uint32_t r = chunk_at[q * (RT / 8) + (tid >> 3)] + ((lower >> (8 * (q & 3))) & 0xFFu);
+#pragma unroll
+        for (int j = 4 * q; j < 4 * q + 4; ++j)
+          if (key[j] == prefix) { m |= r < k_rem ? (1u << j) : 0u; ++r; }
+      }
+    }
   }
+
+  // ---- 2. collect
+#pragma unroll
+  for (int j = 0; j < KPT; ++j) m |= (key[j] != 0u && (tied ? key[j] > prefix : key[j] >= prefix)) ? (1u << j) : 0u;
   uint32_t total = 0u;
   {
     const uint32_t n = (uint32_t)__popc(m);
@@ -994,7 +1077,7 @@ static int launch_radix(const float* logits, int64_t M, int N, int64_t ld, int k
     if (totcap > RMAX_KPAD) totcap = RMAX_KPAD;
   }
   const int lcap = next_pow2(totcap);
-  const size_t smem = (size_t)RCTRL_BYTES + 2 * RBINS * 4 + (size_t)lcap * 8 + (C > 1 ? (size_t)totcap * 8 : 0);
+  const size_t smem = (size_t)RCTRL_BYTES + 2 * RBINS * 4 + 2 * RCHUNKS * 4 + (size_t)lcap * 8 + (C > 1 ? (size_t)totcap * 8 : 0);
   const int vec_ok = (N % 4 == 0) && (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   auto kernel = slice <= 8 * RT ? topk_radix_kernel<8> : (slice <= 16 * RT ? topk_radix_kernel<16> : topk_radix_kernel<32>);
   MOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
