@@ -1,7 +1,11 @@
 """Arguments that the front end has to refuse before the library sees them.  Runs on CPU: the library is replaced by one
 that must not be reached, and the tensors pass for CUDA tensors."""
+import subprocess
+import sys
+
 import pytest
 import torch
+from conftest import ROOT
 
 from tilelang_moe_b200 import ops
 
@@ -33,3 +37,16 @@ def test_routed_gemm_wants_one_device(no_library):
     for args in ((X, W.to("meta"), ids), (X, W, ids.to("meta"))):
         with pytest.raises(ValueError, match="one device"):
             ops.grouped_gemm_routed(*args, 1)
+
+
+def test_import_under_a_torch_without_cuda():
+    """The private functions behind the current device and stream are missing there: the module loads all the same and
+    refuses CPU tensors with its message."""
+    code = ("import torch\n"
+            "for name in ('_cuda_getDevice', '_cuda_getCurrentRawStream'):\n"
+            "    if hasattr(torch._C, name): delattr(torch._C, name)\n"
+            "from tilelang_moe_b200 import ops\n"
+            "try: ops.topk_softmax(torch.zeros(2, 8), 2)\n"
+            "except ValueError as e: print(e)\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "CUDA tensors only" in r.stdout, r.stderr

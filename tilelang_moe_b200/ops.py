@@ -43,7 +43,10 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
-_getdevice, _rawstream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+# the functions under torch.cuda.current_device() and current_stream(); a torch without CUDA has neither, and only needs to
+# get as far as refusing its tensors
+_getdevice = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+_rawstream = getattr(torch._C, "_cuda_getCurrentRawStream", lambda device: torch.cuda.current_stream(device).cuda_stream)
 _HERE = contextlib.nullcontext()
 
 
