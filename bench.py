@@ -359,10 +359,10 @@ def run_ours(args, wl_name, cfg):
             out_pin.copy_(step(), non_blocking=True)
 
         # kernels per layer.  Shared expert of the routed width and H % 64 == 0 (this workload): router GEMV with its
-        # top-k, histogram (one kernel up to 65536 entries and 1024 experts, else three), up GEMM (gathers its rows,
+        # top-k, histogram (one kernel or three: ops.route_histogram_launches), up GEMM (gathers its rows,
         # shared expert as one more group), down GEMM, combine.  Otherwise: + row gather, + shared up and shared down.
         n1 = T * (k + S)
-        hist = 1 if n1 <= 65536 and E + S <= 1024 else 3
+        hist = ops.route_histogram_launches(n1, E + S)
         ride = S == 1 and H % 64 == 0
         launches_per_step = 1 + hist + 2 + 1 + (0 if ride else (2 * (S > 0) + (H % 64 != 0)))
         tokens_per_step = T
@@ -381,7 +381,7 @@ def run_ours(args, wl_name, cfg):
             scores, idx32 = ops.topk_softmax(logits, k, mode="A", index_dtype=torch.int32)
             return layer.routed_forward(x, scores, idx32, Wg, Wu, Wd, ws, timers=timers)
 
-        hist = 1 if T * k <= 65536 and E <= 1024 else 3
+        hist = ops.route_histogram_launches(T * k, E)
         launches_per_step = 4 + hist + (0 if ws.fused_gather else 1)   # topk, histogram, [gather,] up, down, combine
         x_pin = x_cpu.pin_memory()
         lg_pin = logits_cpu.pin_memory()

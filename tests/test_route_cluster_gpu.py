@@ -37,3 +37,10 @@ def test_ids_outside_the_range_are_left_out(cuda, lib):
     assert n == int(keep.sum())
     where = torch.nonzero(keep).view(-1)
     assert torch.equal(perm[:n].cpu().long(), where[torch.argsort(ids[keep], stable=True)])
+
+
+@pytest.mark.parametrize("n", [32768, 32769, 49152, 65535])
+@pytest.mark.parametrize("E", [128, 129])
+def test_one_launch_or_three(cuda, lib, n, E):
+    """Either side of the rule that leaves few experts of a long list to the three kernels."""
+    test_cluster_histogram(cuda, lib, n, E)

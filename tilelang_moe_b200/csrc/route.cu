@@ -24,8 +24,8 @@ constexpr int RUNIT = 1024;        // entries per warp (large inputs)
 constexpr int RUNIT_SMALL = 128;   // entries per warp when the whole input is small: more warps, shorter serial walks
 constexpr int64_t RSMALL_MAX = 65536;    // up to here the three kernels cut the list into the small units (one warp each) ...
 constexpr int64_t RSMALL_TABLE = 131072; // ... as long as the units x experts table the scan kernel walks stays this small
-// measured inside a CUDA graph, E = 256 (us, small / large units): n = 32768 18 / 36, 65536 30 / ~45; beyond that the
-// table walk of the scan kernel outweighs the extra warps (n = 262144: 90 with small units, 524288: 57 with large)
+// measured inside a CUDA graph, E = 1025 (us, small / large units): n = 1000 14.1 / 35.9, 4096 22.7 / 35.5, 8192 34.5 / 38.0, 16000
+// 60.2 / 39.7; for up to 1024 experts the three kernels run above 32768 entries only (route_histogram_ex)
 __host__ __device__ inline bool route_small_units(int64_t n, int E) {
   return n <= RSMALL_MAX && ((n + RUNIT_SMALL - 1) / RUNIT_SMALL) * (int64_t)E <= RSMALL_TABLE;
 }
@@ -198,7 +198,7 @@ route_scatter_kernel(const void* __restrict__ ids, int is64, int64_t n, int E, c
 // register.  Then the counts are summed, over the warps of the CTA, over the CTAs of the cluster (distributed shared
 // memory) and over the experts, and every entry's place is three look-ups.  Same results as the three kernels above.
 // What bounds it: latency.  Measured inside a graph (us, one CTA up to 2048 or 4096 entries and three kernels above -> this):
-// n = 3072, E = 9 6.0 -> 5.1; 4096, 64 10.4 -> 5.7; 8192, 8 9.2 -> 4.6; 32768, 256 17.9 -> 11.4; 65536, 256 29.5 -> 20.1.
+// n = 3000, E = 9 5.9 -> 4.7; 4096, 64 10.5 -> 5.8; 8192, 8 8.7 -> 4.8; 32768, 256 17.4 -> 11.8; 65536, 256 27.6 -> 20.4.
 template <int ROUNDS>
 __global__ void __launch_bounds__(1024)
 route_cluster_kernel(const void* __restrict__ ids, int is64, int n, int E, const int32_t* __restrict__ id_map,
@@ -233,8 +233,9 @@ route_cluster_kernel(const void* __restrict__ ids, int is64, int n, int E, const
 #pragma unroll
   for (int r = 0; r < ROUNDS; ++r) {
     const bool valid = e[r] >= 0;
-    // lanes without a valid id get a private group so that they match nobody
-    const unsigned grp = __match_any_sync(0xFFFFFFFFu, valid ? (unsigned)e[r] : (0x80000000u | (unsigned)lane));
+    // lanes without a valid id share one value: the instruction takes as long as there are different ones in the warp, and
+    // most of the last CTA may have none (us, a value for each of them -> this: 24000 entries, 8 experts 9.4 -> 6.5)
+    const unsigned grp = __match_any_sync(0xFFFFFFFFu, valid ? (unsigned)e[r] : 0xFFFFFFFFu);
     const int rank = __popc(grp & lt_mask);
     const int32_t base = valid ? wh[e[r]] : 0;
     pos[r] = base + rank;
@@ -692,7 +693,11 @@ int moe::route_histogram_ex(const void* topk_idx, int idx_is_int64, int64_t n, i
     const int64_t m = v ? atoll(v) : RCLUSTER_MAX;
     return m < RCLUSTER_MAX ? m : RCLUSTER_MAX;
   }();
-  if (n <= single_max && n > 0 && E <= 1024) {
+  // Above 32768 entries a thread holds eight, and with few experts, where a warp's ids are seldom alike, the rounds of
+  // match.any outlast the three kernels.  Measured (us, three kernels / one launch): 32768 entries: E = 17 9.5 / 7.9, 64
+  // 10.7 / 10.4, 128 12.0 / 11.1; 40000: 17 10.1 / 13.7, 64 11.4 / 18.1, 128 14.5 / 19.3, 129 19.1 / 19.5, 256 21.5 / 20.2;
+  // 60000: 64 12.8 / 18.2, 100 22.0 / 19.2, 128 18.2 / 19.5, 129 28.5 / 19.5, 256 28.2 / 20.2.
+  if (n <= single_max && n > 0 && E <= 1024 && (n <= RCLUSTER_MAX / 2 || E > 128 || (E > 64 && n > 7 * 8192))) {
     // as many CTAs as give every thread one entry; above 8192 entries more entries per thread
     int C = 1;
     while (C < 8 && n > C * 1024) C <<= 1;

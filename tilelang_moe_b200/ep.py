@@ -498,6 +498,7 @@ class EPRunner:
             bufs["out"] = outd
             self.forward(xd, lgd)
 
+        from . import ops
         from .pipeline import HostPipeline
         pipe = HostPipeline(dev, [x_pin, lg_pin], (Tl, x_l.shape[1]), torch.bfloat16, compute, depth=3)   # uploads run two steps ahead
 
@@ -509,5 +510,5 @@ class EPRunner:
         d2h = out_pin.numel() * 2 * self.world
         # peer exchange: topk, histogram, [unique,] histogram exchange, plan, dispatch, barrier, up, down (+ scatter),
         # barrier, combine; NCCL variant: topk, histogram, gather, regroup, gather, up, down, combine
-        hist = 1 if self.Tl * self.cfg["k"] <= 65536 and self.plan.n_slots <= 1024 else 3
+        hist = ops.route_histogram_launches(self.Tl * self.cfg["k"], self.plan.n_slots)
         return step, step_e2e, ((10 if self.px.dedup else 9) if self.px is not None else 7) + hist, h2d, d2h

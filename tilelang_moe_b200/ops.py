@@ -154,6 +154,11 @@ def route_histogram(topk_idx: torch.Tensor, n_experts: int, want_perm: bool = Tr
     return counts, offsets, perm, inv
 
 
+def route_histogram_launches(n: int, n_experts: int) -> int:
+    """Kernels that route_histogram launches for n entries (the library's rule, restated for launch counts)."""
+    return 1 if n_experts <= 1024 and (0 < n <= 32768 or (n <= 65536 and (n_experts > 128 or (n_experts > 64 and n > 57344)))) else 3
+
+
 def gather_rows(src: torch.Tensor, perm: Optional[torch.Tensor], div: int = 1, out: Optional[torch.Tensor] = None,
                 w_src: Optional[torch.Tensor] = None, w_out: Optional[torch.Tensor] = None, n_rows: Optional[int] = None):
     """out[p] = src[perm[p] // div]; optionally w_out[p] = w_src[perm[p]]."""
