@@ -175,3 +175,9 @@ def test_silu_over_its_whole_range(cuda, lib, monkeypatch, form):
     far = gate.isfinite() & (gate < -88.65)
     assert far.any() and bool(((y[:, far] <= 0) & (y[:, far] > -1e-35)).all())
     assert bool((y[:, gate == float("inf")] == float("inf")).all()) and bool(y[:, ~gate.isfinite() & (gate != float("inf"))].isnan().all())
+
+
+@pytest.mark.parametrize("T,H,E,k", [(7, 1016, 16, 2), (7, 1024, 16, 2), (40, 256, 9, 3), (40, 256, 8, 3), (40, 256, 17, 3)])
+def test_a_cta_or_a_warp_per_token_of_short_rows(cuda, lib, T, H, E, k):
+    """... and on the sides of its rule on the hidden size and the number of experts."""
+    test_few_experts_a_cta_or_a_warp_per_token(cuda, lib, T, H, E, k, torch.bfloat16)

@@ -800,9 +800,12 @@ static int router_small(const void* x, const void* Wr, int64_t T, int H, int E, 
   if (rc) return rc;
   const size_t smem = (size_t)E * H * 2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // Measured (us, H = 2048, E = 8): 8 tokens 6.8 with a warp per token, 3.4 with a CTA; 1024 tokens 7.2 either way, and the
-  // weight is read from L2 for every token: a CTA per token up to two per SM
-  if (T <= (int64_t)dev.sm_count * 2) {
+  // A CTA per token up to two per SM: from there on the weight, read from L2 for every token, costs some shapes more than the
+  // staging saves.  Measured (us, a warp per token / a CTA per token): 8 tokens, E = 8, H = 256 3.4 / 3.3, H = 2048 6.8 / 3.6;
+  // 296 tokens, E = 16, H = 512 5.5 / 5.8, 1024 7.2 / 5.9; E = 32, H = 256 7.2 / 7.1, 2048 20.1 / 7.7; 592 tokens, H = 1024, E = 8
+  // 5.1 / 3.8, H = 256, E = 32 7.3 / 9.5; 1024 tokens, E = 8, H = 1024 5.1 / 5.9, 2048 6.8 / 6.9.  Nine to sixteen experts
+  // on short rows keep the warp: 8 tokens, E = 16, H = 256 4.4 / 5.4.
+  if (T <= (int64_t)dev.sm_count * 2 && (H >= 1024 || E <= 8 || E > 16)) {
 #define MOE_RT_LAUNCH(F16_, EMAX_)                                                                                       \
     router_token_kernel<F16_, EMAX_><<<(unsigned)T, 256, 0, st>>>(reinterpret_cast<const uint4*>(x),                     \
         reinterpret_cast<const uint4*>(Wr), H / 8, E, logits, k, mode, scores, idx64, idx32)
