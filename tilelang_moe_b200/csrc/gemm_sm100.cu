@@ -904,24 +904,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           uint32_t va[32], vb[32];
           tmem_ld32(taddr + c * 64, va);
           tmem_ld32(taddr + c * 64 + 32, vb);
-          if (EPI == MOE_GEMM_SILU_GATE) {
-            uint32_t ua[32], ub[32];
-            tmem_ld32(taddr + BN / 2 + c * 64, ua);
-            tmem_ld32(taddr + BN / 2 + c * 64 + 32, ub);
-            tmem_ld_wait();
+          tmem_ld_wait();
+          if (EPI == MOE_GEMM_SCALE_SCATTER) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-              va[j] = __float_as_uint(silu_mul(__uint_as_float(va[j]), __uint_as_float(ua[j])));
-              vb[j] = __float_as_uint(silu_mul(__uint_as_float(vb[j]), __uint_as_float(ub[j])));
-            }
-          } else {
-            tmem_ld_wait();
-            if (EPI == MOE_GEMM_SCALE_SCATTER) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                va[j] = __float_as_uint(__uint_as_float(va[j]) * w);
-                vb[j] = __float_as_uint(__uint_as_float(vb[j]) * w);
-              }
+              va[j] = __float_as_uint(__uint_as_float(va[j]) * w);
+              vb[j] = __float_as_uint(__uint_as_float(vb[j]) * w);
             }
           }
           uint4* mine = reinterpret_cast<uint4*>(stg + lane * C::STAGING_PITCH);
