@@ -181,3 +181,27 @@ def test_silu_over_its_whole_range(cuda, lib, monkeypatch, form):
 def test_a_cta_or_a_warp_per_token_of_short_rows(cuda, lib, T, H, E, k):
     """... and on the sides of its rule on the hidden size and the number of experts."""
     test_few_experts_a_cta_or_a_warp_per_token(cuda, lib, T, H, E, k, torch.bfloat16)
+
+
+@pytest.mark.parametrize("K,N", [(64, 8), (128, 200), (192, 512)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_epilogue_of_few_and_many_rows_per_warp(cuda, lib, K, N, dtype):
+    """Groups that end in warps of 1 to 32 rows, 64-row and 128-row tiles: rows stored directly and through shared memory, scattered
+    and scaled.  Inputs on a coarse grid make every sum exact in fp32, so the result is its one rounding."""
+    sizes = [1, 2, 15, 16, 17, 31, 32, 33, 48, 49, 0, 64, 65, 79, 80, 81, 97, 112, 113, 127, 128, 129, 145]
+    E, n = len(sizes), sum(sizes)
+    g = torch.Generator().manual_seed(K + N)
+    A = (torch.randn(n, K, generator=g) * 2).round().clamp(-4, 4).to(dtype)
+    W = ((torch.randn(E, N, K, generator=g) * 2).round().clamp(-4, 4) / 8).to(dtype)
+    offs = torch.tensor([0, *sizes]).cumsum(0).int()
+    dst = torch.randperm(n, generator=g).int()
+    w = torch.randint(1, 9, (n,), generator=g).float() / 4
+    y = torch.cat([A[a:b].float() @ W[e].float().T for e, (a, b) in enumerate(zip(offs[:-1].tolist(), offs[1:].tolist()))])
+    dev = [t.to(cuda) for t in (A, W, offs, dst, w)]
+    want = torch.empty(n, N, dtype=dtype)
+    want[dst.long()] = y.to(dtype)
+    assert torch.equal(ops.grouped_gemm_sorted(ops.GEMM_PLAIN, dev[0], dev[1], dev[2], dst_rows=dev[3]).cpu(), want)
+    want[dst.long()] = (y * w[:, None]).to(dtype)
+    got = ops.grouped_gemm_sorted(ops.GEMM_SCALE_SCATTER, dev[0], dev[1], dev[2], dst_rows=dev[3], row_w=dev[4])
+    assert torch.equal(got.cpu(), want)
+    ops.check_status(cuda)

@@ -886,13 +886,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       // 16-bit rows leave 64 columns at a time through shared memory (this warp's 32 rows x 128 bytes), 8 lanes per row:
       // a store instruction then carries four 128-byte row segments instead of thirty-two 16-byte pieces of as many rows.
       // Measured with %globaltimer stamps (1024 tokens, 9 experts, N = 2048, scale + scatter): 3.65 us per 128 x 256 tile with
-      // direct stores and the rows looked up after the accumulator was ready, 2.9-3.1 now.  Calls: grouped GEMM of 8192 rows,
-      // H = 7168, I = 2048, 32 experts 344 -> 337 us; layer of 1024 tokens 59.4 -> 58.5.  SiLU tiles keep the direct form:
-      // 128 columns leave a tile, and staging them measured 2.8 against 2.2 us.
+      // direct stores and the rows looked up after the accumulator was ready, 2.9-3.1 now.  2048 rows on 8 experts, K = 512,
+      // N = 2048: 17.6 -> 15.6 us; with long K it hides behind the main loop (8192 rows on 32 experts, K = 7168: no difference beyond
+      // noise).  SiLU tiles keep the direct form: 128 columns leave a tile, and staging them measured 2.8 against 2.2 us.
       constexpr bool STAGED = EPI != MOE_GEMM_PLAIN_F32 && EPI != MOE_GEMM_SILU_GATE;
       const unsigned live = __ballot_sync(0xFFFFFFFFu, row_ok);
       const int span = 32 - __clz(live);            // rows of this warp up to its last live one
-      if (STAGED) {
+      // Up to 16 rows store directly: staging takes a warp as long for one row as for 32, and a warp of an M = 64 tile (groups of
+      // few rows) never has more than 16.  Measured (us, gathered plain GEMM;
+      // direct / staged / this): 1024 rows on 64 experts, K = 128, N = 1024: 9.0 / 10.5 / 8.9; 2048 rows 9.2 / 10.9 / 9.4; 100 rows on
+      // 8 experts, K = 512, N = 2048: 7.9 / 8.8 / 8.3.
+      if (STAGED && (EPI == EPI_PEER || span > 16)) {
         unsigned char* stg = smem + C::STAGING_OFFSET + (warp - 2) * 32 * C::STAGING_PITCH;
         const unsigned long long row_ptr = row_ok
             ? reinterpret_cast<unsigned long long>(reinterpret_cast<__nv_bfloat16*>(ybase) + out_row * p.ldy) : 0ull;
@@ -944,6 +948,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(silu_mul(__uint_as_float(v[j]), __uint_as_float(u[j])));
           } else {
             tmem_ld_wait();
+            if (EPI == MOE_GEMM_SCALE_SCATTER) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * w);
+            }
           }
           const int col = n0 + c * 32;
           if (row_ok && col < p.N) {
