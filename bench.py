@@ -1024,7 +1024,7 @@ def run_router(args):
         s2, i2 = two()
         row["same_indices"] = bool(torch.equal(i1, i2))
         row["default_rule_picks"] = ("split_k" if (ops.router_splits(T, H) >= 4 and not (E <= 32 and E * H * 2 <= 200 * 1024))
-                                     else ("one_kernel" if (E <= 64 or T >= 32 * E) else "two_kernels"))
+                                     else ("one_kernel" if ops.router_one_kernel(T, E) else "two_kernels"))
         byts = (T * H + E * H) * 2 + T * K * 12
         row["GBps_one_kernel"] = round(byts / row["us_one_kernel"] / 1e3, 1)
         row["frac_hbm_measured"] = round(byts / row["us_one_kernel"] / 1e3 / peaks["hbm_gbs"], 3)

@@ -205,3 +205,16 @@ def test_epilogue_of_few_and_many_rows_per_warp(cuda, lib, K, N, dtype):
     got = ops.grouped_gemm_sorted(ops.GEMM_SCALE_SCATTER, dev[0], dev[1], dev[2], dst_rows=dev[3], row_w=dev[4])
     assert torch.equal(got.cpu(), want)
     ops.check_status(cuda)
+
+
+@pytest.mark.parametrize("T,E", [(4095, 128), (4096, 128), (9472, 136), (9473, 136), (700, 64)])
+def test_router_on_the_sides_of_its_rule(cuda, lib, T, E):
+    """One kernel or two, as the rule picks: the same logits, so the same scores and indices."""
+    g = torch.Generator().manual_seed(T)
+    X, W = torch.randn(T, 64, generator=g).bfloat16().to(cuda), torch.randn(E, 64, generator=g).bfloat16().to(cuda)
+    s, i = ops.router_topk_softmax(X, W, 6, mode="A")
+    ops.check_status(cuda)
+    for fused in (True, False):
+        s2, i2 = ops.router_topk_softmax(X, W, 6, mode="A", fused=fused)
+        assert torch.equal(i, i2)
+        torch.testing.assert_close(s, s2, rtol=2e-6, atol=0)

@@ -210,7 +210,8 @@ extern "C" int moe_layer_forward_ex(const void* x, const void* router_weight, co
     rc = moe_topk_softmax(logits, T, E, E, k, MOE_TOPK_MODE_A, scores, nullptr, idx32, status, stream);
     if (rc) return leave(rc);
   } else {
-    // one kernel when the shape allows and has enough row tiles to hide the selection, else GEMM then top-k
+    // one kernel when the shape allows and has enough row tiles to hide the selection, else GEMM then top-k (both sides
+    // measured: router_one_kernel in ops.py; 148 SMs)
     const bool small = E <= 32 && (size_t)E * H * 2 <= 200 * 1024;
     const int splits = router_splits(T, H);
     if (!small && splits >= 4 && E % 8 == 0 && E >= 8 && E <= 256 && k <= 32) {
@@ -220,7 +221,7 @@ extern "C" int moe_layer_forward_ex(const void* x, const void* router_weight, co
       if (rc) return leave(rc);
       goto routed;
     }
-    const bool fused = small || (E % 8 == 0 && E >= 8 && E <= 256 && k <= 8 && (E <= 64 || T >= 32 * (int64_t)E));
+    const bool fused = small || (E % 8 == 0 && E >= 8 && E <= 256 && k <= 8 && (E <= 64 || (E <= 128 ? T >= 32 * (int64_t)E : T > 64 * 148)));
     if (fused) {
       rc = moe_router_topk(x, router_weight, T, H, E, k, MOE_TOPK_MODE_A, dtype, scores, nullptr, idx32, nullptr, status, stream);
       if (rc) return leave(rc);

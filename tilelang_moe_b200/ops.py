@@ -337,6 +337,18 @@ def router_splits(T: int, H: int) -> int:
     return S
 
 
+def router_one_kernel(T: int, E: int) -> bool:
+    """Whether the router runs as one kernel, or as a GEMM and a top-k kernel (the library's rule, restated).
+
+    With few row tiles nothing hides the selection in the epilogue, and the separate top-k kernel, on all SMs, is
+    quicker; above 128 experts the GEMM has two column tiles per row tile, and the two kernels stay ahead while these
+    fit the SMs at once (64 tokens per SM).  Measured on a B200 (us, one kernel / two): H = 7168, k = 8, E = 64:
+    5000 tokens 44.9 / 43.8, 16384 49.8 / 52.0; E = 128: 5000 46.3 / 44.4, 8192 46.6 / 46.1, 16384 52.3 / 55.0; E = 256: 8192
+    53.3 / 48.5, 12345 54.8 / 85.1, 16384 58.4 / 94.5; H = 1024, k = 2, E = 64: 5000 12.4 / 13.3; E = 96: 5000 13.3 / 15.2;
+    E = 160: 8192 16.2 / 17.0, k = 8 18.7 / 18.0, 12345 19.1 / 22.6."""
+    return E <= 64 or (T >= 32 * E if E <= 128 else T > 64 * 148)
+
+
 def _router_topk_splitk(x, router_weight, k, mode, index_dtype, logits_out):
     T, H = x.shape
     E = router_weight.shape[0]
@@ -374,14 +386,11 @@ def router_topk_softmax(x: torch.Tensor, router_weight: torch.Tensor, k: int, mo
     E = router_weight.shape[0]
     small_e = E <= 32 and E * H * 2 <= 200 * 1024
     if fused is None:
-        # Measured on B200: with few row tiles the selection in the epilogue is not hidden behind another tile's
-        # main loop, and the separate top-k kernel (all SMs) is quicker; from about 32 tokens per expert the single
-        # kernel wins (T=16384: 93 vs 124 us at E=256, 44 vs 48 us at E=64).  Few experts: always one kernel.
         # Few tokens (at most a quarter of the SMs would get a row tile): the GEMM is split along K instead.
         if not small_e and router_splits(T, H) >= 4 and E % 8 == 0 and 8 <= E <= 256 and k <= 32:
             fused = "splitk"
         else:
-            fused = E <= 64 or T >= 32 * E
+            fused = router_one_kernel(T, E)
     if fused == "splitk":
         return _router_topk_splitk(x, router_weight, k, mode, index_dtype, logits_out)
     if not fused or not router_topk_fused_supported(H, E, k) or T == 0:
