@@ -438,21 +438,21 @@ __device__ __forceinline__ uint4 pack_out8(const uint32_t* v, int f16) {
 // g * sigmoid(g) * u.  The quotient g / d, d = 1 + exp(-g), comes from an approximate reciprocal (1 ulp) and one step of
 // Newton's iteration on the quotient with the remainder in one fma (Markstein, IBM J. Res. Dev. 34, 1990): the nearest fp32
 // but for ties within 2^-45 (4 Mi gates in each of seven ranges of [-88.7, 1e4]: the bits of the checked division in all of
-// them, 0.5 ulp at most; the fast intrinsic has 2, and zero where d exceeds 2^126, from g = -87.3 on).  The reciprocal is
-// taken of d / 4, or it would be flushed to zero there.  The remainder is NaN where g or d is infinite: the first quotient stands.
+// them, 0.5 ulp at most; the fast intrinsic has 2, and zero where d exceeds 2^126, from g = -87.3 on).  Everything is done on
+// d / 4 and g / 4, or the reciprocal would be flushed to zero there; gates below 2^-124 lose a unit of 2^-149 by that.  The
+// remainder is NaN where g or d is infinite: the first quotient stands.
 // No branch: the checked division leaves its fast path for extreme values, element by element, while the whole warp waits -
 // lanes without a live row hold whatever tensor memory held - and its call costs live rows alone nearly as much.
 // Measured, up GEMM (us; checked in all lanes / in live rows / fast intrinsic / this): 16 rows on 9 experts, H = 2048,
-// I = 512: 39.3 / 17.4 / 15.8 / 16.1; 2048 rows 39.4 / 24.0 / 18.0 / 18.4; 8192 rows on 8 experts, H = 512, I = 2048:
-// 118.8 / 79.4 / 42.0 / 43.2.
+// I = 512: 39.3 / 17.4 / 15.8 / 16.0; 2048 rows 39.4 / 24.0 / 18.4 / 18.3; 8192 rows on 8 experts, H = 512, I = 2048:
+// 118.8 / 79.4 / 42.3 / 43.1.
 __device__ __forceinline__ float silu_mul(float g, float u) {
-  const float d = 1.0f + __expf(-g);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(0.25f * d));
-  r *= 0.25f;
-  const float q = g * r;
-  const float rem = fmaf(-d, q, g);
-  return (fabsf(rem) > 0.0f ? fmaf(rem, r, q) : q) * u;
+  const float d4 = fmaf(__expf(-g), 0.25f, 0.25f), g4 = 0.25f * g;
+  float r4;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r4) : "f"(d4));
+  const float q = g4 * r4;
+  const float rem4 = fmaf(-d4, q, g4);
+  return (fabsf(rem4) > 0.0f ? fmaf(rem4, r4, q) : q) * u;
 }
 
 // One row of router logits per thread, N of them (N % 8 == 0, at most 256) in tensor-memory columns taddr ...: top-k,
