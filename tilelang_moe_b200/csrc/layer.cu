@@ -54,8 +54,13 @@ static LayerScratch layer_layout(int64_t T, int k, int H, int I, int E, int SI) 
   return L;
 }
 
-// Overlapping a kernel's start with the end of the one before it hides a few us per boundary, whatever the size; the
-// kernels of a long batch last a hundred times that, and CTAs that wait beside them only take their room.
+// Overlapping a kernel's start with the end of the one before it hides a us or two per call, whatever the size; the kernels
+// of a long batch last a hundred times that, and CTAs that wait beside them take their room.  Measured (us, plain launches /
+// dependent): 8 experts, H = 256, I = 128, k = 1, shared: 1024 tokens 29.1 / 27.9, 4096 36.1 / 35.1, 16384 76.5 / 75.6; 16, H = 1024,
+// I = 128, k = 4: 1024 49.7 / 46.9, 4096 93.7 / 92.8, 16384 255 / 256; 256, H = 1024, I = 256, k = 8: 2048 129.6 / 127.2, 4096
+// 169.3 / 170.8, 8192 243 / 250; 128, H = 1000, I = 256, k = 8: 4096 187.0 / 188.1, 6000 230 / 237, 16384 524 / 553.
+// moe_grouped_gemm_routed, two or three kernels, launches dependently at any size: 64 to 32768 tokens of six shapes gain up to
+// 1 us and lose nothing beyond noise (8 experts, H = 1024, I = 256, k = 2: 1024 tokens 16.0 / 14.9, 32768 49.4 / 48.8).
 constexpr int64_t PDL_MAX_TOKENS = 4096;
 
 struct RoutedScratch {
