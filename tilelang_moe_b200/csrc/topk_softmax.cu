@@ -151,14 +151,16 @@ static int launch_warp(const float* logits, int64_t M, int N, int64_t ld, int k,
 //      entries (equal keys: lowest column first);
 //   3. each lane ranks its share of them against all of them; the entries of rank < k are the result, in order.
 // NaNs do not enter V (max and min ignore them) and are never below it, so they are collected and rank first by key.
-// A warp with more than CAP entries in one of its rows takes the logits equal to V in column order, K at most; where
-// the logits above V alone are too many (rows sorted by expert, rows masked to -inf), every lane keeps a sorted list.
+// A warp with more than CAP entries in one of its rows takes the logits equal to V in column order, as many as those above V
+// leave of K; where the logits above V alone are too many (rows sorted by expert), every lane keeps a sorted list.
 //
 // What bounds it: instruction issue at N = 128, HBM from N = 512 on.  Few rows: the chain of one warp.  Measured (us,
-// thread-per-row tiles with a list of K per thread before -> now): 1048576 x 128, k = 6: 169 -> 138 (HBM 92);
-// 131072 x 256, k = 8: 65 -> 34; 131072 x 1024, k = 8: 291 -> 122 (HBM 83); 16384 x 256: 13.0 -> 7.9; 2048 x 256:
-// 9.0 -> 3.4; 131072 x 128 with all logits equal 24.6 -> 20.6, rounded to integers 28.7 -> 25.7.  With a few lanes per
-// row 32 warps per SM fit beside each other; the tiles had 12.
+// thread-per-row tiles with a list of K per thread before -> now): 1048576 x 128, k = 6: 169 -> 138 (HBM 93);
+// 131072 x 256, k = 8: 65.7 -> 34.3; 131072 x 1024, k = 8: 291 -> 115 (HBM 84); 16384 x 256: 11.7 -> 6.8; 2048 x 256:
+// 8.8 -> 3.4.  With a few lanes per row 32 warps per SM fit beside each other; the tiles had 12.  Equal logits: 131072 x
+// 128, k = 6 all equal 25.0 -> 21.4, rounded to integers 29.0 -> 24.2; rounded, k = 8: 32768 x 128 13.2 -> 11.2, 131072 x 64
+// 33.0 -> 20.9.  Slower than the tiles and the warp kernel: rounded to integers, k = 2, 32768 x 36 4.8 -> 6.2, x 100 6.1 -> 6.8 (a
+// dozen entries to rank for two places), and 64 x 300, k = 8 3.9 -> 4.5.
 // ------------------------------------------------------------------------------------
 constexpr int GROUP_WARPS = 8;
 
@@ -266,7 +268,8 @@ topk_group_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
   int c = __shfl_sync(FULL, inc, L - 1, L);
   int cmax = __reduce_max_sync(FULL, c);
   if (cmax > CAP) {
-    // many logits equal to V: collect those above it and, one column at a time, the first K of the equal ones
+    // many logits equal to V: collect those above it and, where these are fewer than K, the first of the equal ones, one
+    // column at a time
     uint32_t eq = 0u;
 #pragma unroll
     for (int b = 0; b < EPT; ++b) eq |= x[b] == V ? (1u << b) : 0u;
@@ -281,15 +284,16 @@ topk_group_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
     }
     c = __shfl_sync(FULL, inc, L - 1, L);
     cmax = __reduce_max_sync(FULL, c);
-    if (cmax <= CAP - K) {
+    if (cmax <= CAP) {
       const uint64_t vkey = (uint64_t)float_to_key(V) << 32;
-      for (int r = 0; r < K; ++r) {
+      const int rounds = __reduce_max_sync(FULL, K - c);
+      for (int r = 0; r < rounds; ++r) {
         const int b = __ffs(eq) - 1;
         const uint32_t col = eq ? (uint32_t)(4 * ((b >> 2) * L + sub) + (b & 3)) : 0xFFFFFFFFu;
         uint32_t first = col;
 #pragma unroll
         for (int d = 1; d < L; d <<= 1) first = min(first, __shfl_xor_sync(FULL, first, d));
-        if (first != 0xFFFFFFFFu) {
+        if (first != 0xFFFFFFFFu && c < K) {
           if (col == first) {
             cand[c] = vkey | (uint64_t)(0xFFFFFFFFu - col);
             eq &= eq - 1;
@@ -432,7 +436,7 @@ static int launch_group(const float* logits, int64_t M, int N, int64_t ld, int k
 // indices leave through shared memory as contiguous runs of the warp's 32 rows.
 //
 // What bounds it: the stores and the lists.  Measured (us, thread-per-row tiles before -> now): 1048576 x 16, k = 2:
-// 63 -> 30; 1048576 x 8: 59 -> 27; 16384 x 16: 3.6 -> 2.5.  (The same form for 128 logits: 132 us for 1048576 rows
+// 58.8 -> 26.7; 1048576 x 8: 54.7 -> 24.8; 16384 x 16: 3.7 -> 2.6; all logits equal, 32768 x 32, k = 2: 4.3 -> 4.9.  (The same form for 128 logits: 132 us for 1048576 rows
 // against 140 with four lanes per row, but twice its time on tied logits, and 6.7 against 4.9 us for 16384 rows: not built.)
 // ------------------------------------------------------------------------------------
 constexpr int LANE_WARPS = 4;
