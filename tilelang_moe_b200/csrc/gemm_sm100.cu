@@ -2,8 +2,8 @@
 //
 //   Y[rows of expert e] = A[rows of expert e] . B[e]^T          (A: [rows,K], B: [E,N,K], K contiguous)
 //
-// One persistent CTA per SM, 256 threads in four roles (192 threads and the first three roles in the CTA-pair and
-// tokens-as-N kernels):
+// One persistent CTA per SM, 256 threads in four roles (192 threads and the first three roles without a row gather and in
+// the CTA-pair kernel):
 //   warp 0      TMA producer: per k-block one A box (128 rows x 64) and the B box(es) (BN rows x 64),
 //               128-byte swizzled, into a ring of shared-memory stages guarded by mbarriers;
 //   warp 1      MMA issuer: one thread issues tcgen05.mma (M=128, N=BN, K=16) four times per
@@ -11,13 +11,10 @@
 //               the accumulator.  Also owns the TMEM allocation;
 //   warps 2..5  epilogue: tcgen05.ld the fp32 accumulator, apply the fused epilogue, store 16-byte
 //               vectors with row masks;
-//   warps 6..7  row gather (see below); idle otherwise.
+//   warps 6..7  row gather (see below).
 //
-// Two tile shapes.  MT=1: 128 rows x BN columns, accumulator double-buffered in TMEM so that the next
-// tile's main loop overlaps the epilogue.  MT=2: 256 rows x 256 columns as two M=128 MMAs per K step
-// that share one B tile in shared memory - a third less operand traffic into the SM per flop, which is
-// what limits the MT=1 shape (all 512 TMEM columns hold one tile, so the epilogue is not overlapped).
-// A tile whose expert has no more than 128 rows left issues only the first of the two MMAs.
+// Tiles of 128 rows x BN columns, accumulator double-buffered in TMEM so that the next tile's main loop overlaps the
+// epilogue; tiles of 256 rows, which bring a third less operand traffic into the SM per flop, are the CTA-pair kernel's.
 //
 // Tiles are enumerated on the device from the expert offsets (no host sync): expert-major, then
 // N tile, then M tile, so that CTAs running side by side share one B tile through L2.
@@ -72,16 +69,15 @@ constexpr uint64_t DRAIN_LIMIT_NS = 20ull * 1000ull * 1000ull;    // 20 ms when 
 
 // AR: rows of A a stage holds.  128, or 32 for groups of at most 32 rows: their M = 64 instructions read 64 rows, the
 // upper half from whatever follows in the stage, and nothing of what they make of it is stored.
-template <int MT, int BN, int AR = BM>
+template <int BN, int AR = BM>
 struct Cfg {
-  static constexpr int A_HALF_BYTES = AR * BK * 2;         // one A tile
-  static constexpr int A_BYTES = MT * A_HALF_BYTES;
+  static constexpr int A_BYTES = AR * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (192 * 1024) / STAGE_BYTES;  // 6, 4 or 3; with 32 rows of A 16, 9 or 5
-  static constexpr int ACC_BUFS = (MT * BN * 2 <= 512) ? 2 : 1;
-  static constexpr int TMEM_COLS = ACC_BUFS * MT * BN;       // 128, 256 or 512: powers of two >= 32
-  static_assert(AR == BM || A_HALF_BYTES + B_BYTES >= 64 * BK * 2, "an M = 64 instruction stays inside its stage");
+  static constexpr int STAGES = (192 * 1024) / STAGE_BYTES;  // BN = 128: 6, 256: 4; BN = 64 with 32 rows of A: 16
+  static constexpr int ACC_BUFS = 2;
+  static constexpr int TMEM_COLS = ACC_BUFS * BN;            // 128, 256 or 512: powers of two >= 32
+  static_assert(AR == BM || A_BYTES + B_BYTES >= 64 * BK * 2, "an M = 64 instruction stays inside its stage");
   // layout: [stages][barriers, tensor-memory slot and abort flag 384 B][tile tables]
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int SLOT_OFFSET = BAR_OFFSET + 320;
@@ -471,7 +467,7 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 // 85.8 -> 74.0 -> 61.2; H = 1024, E = 96 22.5 -> 21.8 -> 16.7.  The one loss: logits that ascend with the expert in every
 // row, E = 64 52.7 -> 51.8 -> 53.3.
 constexpr int ROUTER_CAP = 16;
-static_assert((ROUTER_CAP + 1) * 256 <= 32 * Cfg<1, 128>::STAGING_PITCH, "parked logits of a warp fit its staging rows");
+static_assert((ROUTER_CAP + 1) * 256 <= 32 * Cfg<128>::STAGING_PITCH, "parked logits of a warp fit its staging rows");
 __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t taddr, int grow, bool row_ok,
                                                     unsigned char* park, int lane) {
   constexpr int KMAX = 8;
@@ -627,14 +623,14 @@ __device__ __forceinline__ void router_row_epilogue(const Params& p, uint32_t ta
 }
 
 // ------------------------------------------------------------------------------ kernel
-template <int MT, int BN, int EPI, bool GATHER, int AR>
+template <int BN, int EPI, bool GATHER, int AR>
 __global__ void __launch_bounds__(GATHER ? NUM_THREADS_GATHER : NUM_THREADS, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ WeightMap tmB,
                     const __grid_constant__ WeightMap tmB2, const Params p) {
-  using C = Cfg<MT, BN, AR>;
+  using C = Cfg<BN, AR>;
   constexpr int STAGES = C::STAGES;
   constexpr int ACC_BUFS = C::ACC_BUFS;
-  constexpr int TILE_ROWS = MT * BM;
+  constexpr int TILE_ROWS = BM;
   constexpr int OUT_COLS = EPI == MOE_GEMM_SILU_GATE ? BN / 2 : BN;   // output columns per tile
   extern __shared__ unsigned char smem_dyn[];
   // the swizzle pattern needs 1024-byte aligned stage buffers
@@ -740,14 +736,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
       const Tile t = (mixed ? decode_mixed(tile, tstart, lstart, offs, E, NT) : decode_tile(tile, tstart, offs, E, NT, TILE_ROWS));
-      const bool second_half = MT == 2 && (t.row_end - t.row0) > BM;   // rows beyond the first 128 exist
       // a tile with at most 64 live rows is issued as M = 64 instructions: same time per instruction, half the rows
       // switching in the tensor core (what counts under the power cap); its accumulator uses lanes 0..15 of every
       // 32-lane quarter of tensor memory
-      const uint32_t idesc_t = (MT == 1 && p.m64 && t.row_end - t.row0 <= 64) ? idesc64 : idesc;
+      const uint32_t idesc_t = (p.m64 && t.row_end - t.row0 <= 64) ? idesc64 : idesc;
       if (!mbar_wait(tempty0 + 8 * acc, acc_phase ^ 1, abort_flag, p.status, 2)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t d_tmem = tmem_base + (uint32_t)(acc * MT * BN);
+      const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
       for (int kb = 0; kb < NKB; ++kb) {
         if (!mbar_wait(full0 + 8 * stage, phase, abort_flag, p.status, 3)) { ok = false; break; }
         tc_fence_after();
@@ -762,9 +757,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           for (int k = 0; k < BK / UMMA_K; ++k) {
             // advancing K by 16 bf16 = 32 bytes inside the swizzle row: +2 in the (addr >> 4) field
             umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc_t, (kb | k) != 0 ? 1u : 0u);
-            if (second_half)   // rows 128..255 of the tile: next A half (16 KB further), same B, next accumulator
-              umma_bf16(d_tmem + BN, adesc + (uint64_t)(C::A_HALF_BYTES >> 4) + (uint64_t)(2 * k),
-                        bdesc + (uint64_t)(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
           }
           umma_commit(empty0 + 8 * stage);
         }
@@ -845,12 +837,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
       const Tile t = (mixed ? decode_mixed(tile, tstart, lstart, offs, E, NT) : decode_tile(tile, tstart, offs, E, NT, TILE_ROWS));
-#pragma unroll 1
-      for (int half = 0; half < MT; ++half) {
-      if (half == 1 && t.row0 + BM >= t.row_end) break;   // nothing was accumulated for rows 128..255
       // sorted row handled by this thread; an M = 64 tile keeps rows 16q .. 16q+15 in the first 16 lanes of quarter q
-      const bool m64 = MT == 1 && p.m64 && t.row_end - t.row0 <= 64;
-      const int grow = m64 ? t.row0 + q * 16 + lane : t.row0 + half * BM + q * 32 + lane;
+      const bool m64 = p.m64 && t.row_end - t.row0 <= 64;
+      const int grow = m64 ? t.row0 + q * 16 + lane : t.row0 + q * 32 + lane;
       bool row_ok = grow < t.row_end && (!m64 || lane < 16);
       const int n0 = p.ksplit ? 0 : t.n_tile * OUT_COLS;
       int64_t out_row = grow;
@@ -874,12 +863,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         if (EPI == EPI_PEER) ybase = p.peer_base[p.row_rank[grow]];
       }
-      if (half == 0) {   // the rows have been looked up while the main loop was still running
-        if (!mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag, p.status, 4)) { ok = false; break; }
-        tc_fence_after();
-        MOE_TRACE(if (warp == 2 && lane == 0 && tile < MOE_TRACE_MAX_TILES) g_trace_tile[1][tile] = global_timer_ns();)
-      }
-      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * MT * BN + half * BN);
+      // the rows have been looked up while the main loop was still running
+      if (!mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag, p.status, 4)) { ok = false; break; }
+      tc_fence_after();
+      MOE_TRACE(if (warp == 2 && lane == 0 && tile < MOE_TRACE_MAX_TILES) g_trace_tile[1][tile] = global_timer_ns();)
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
       if (EPI == EPI_ROUTER) {
         router_row_epilogue(p, taddr, grow, row_ok, smem + C::STAGING_OFFSET + (warp - 2) * 32 * C::STAGING_PITCH, lane);
       } else {
@@ -971,8 +959,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
       }
       }  // not the router epilogue
-      }  // halves
-      if (!ok) break;
       MOE_TRACE(if (warp == 2 && lane == 0 && tile < MOE_TRACE_MAX_TILES) g_trace_tile[2][tile] = global_timer_ns();)
       tc_fence_before();
       __syncwarp();
@@ -1464,24 +1450,24 @@ static int allow_dynamic_smem(Kernel kernel, int bytes, std::atomic<bool>* done_
   return MOE_OK;
 }
 
-template <int MT, int BN, int EPI, bool GATHER, int AR = BM>
+template <int BN, int EPI, bool GATHER, int AR = BM>
 static int launch_g(const CUtensorMap& tA, const WeightMap& tB, const WeightMap& tB2, const Params& p, int grid,
                     cudaStream_t st) {
-  using C = Cfg<MT, BN, AR>;
+  using C = Cfg<BN, AR>;
   constexpr int SMEM = EPI == MOE_GEMM_PLAIN_F32 || EPI == MOE_GEMM_SILU_GATE ? C::SMEM_BYTES : C::SMEM_BYTES_STAGED;
   static std::atomic<bool> attr_set[64];
-  int rc = allow_dynamic_smem(grouped_gemm_kernel<MT, BN, EPI, GATHER, AR>, SMEM, attr_set);
+  int rc = allow_dynamic_smem(grouped_gemm_kernel<BN, EPI, GATHER, AR>, SMEM, attr_set);
   if (rc) return rc;
-  MOE_LAUNCH("grouped_gemm_kernel", grouped_gemm_kernel<MT, BN, EPI, GATHER, AR>, (unsigned)grid,
+  MOE_LAUNCH("grouped_gemm_kernel", grouped_gemm_kernel<BN, EPI, GATHER, AR>, (unsigned)grid,
              GATHER ? NUM_THREADS_GATHER : NUM_THREADS, SMEM, st, p.pdl != 0, tA, tB, tB2, p);
   return MOE_OK;
 }
-template <int MT, int BN, int EPI>
+template <int BN, int EPI>
 static int launch(const CUtensorMap& tA, const WeightMap& tB, const WeightMap& tB2, const Params& p, int grid,
                   cudaStream_t st) {
   // the row gather is compiled for the matrix epilogues only (the fused router has none)
-  if (EPI != EPI_ROUTER && p.a_gather) return launch_g<MT, BN, EPI == EPI_ROUTER ? MOE_GEMM_PLAIN : EPI, true>(tA, tB, tB2, p, grid, st);
-  return launch_g<MT, BN, EPI, false>(tA, tB, tB2, p, grid, st);
+  if (EPI != EPI_ROUTER && p.a_gather) return launch_g<BN, EPI == EPI_ROUTER ? MOE_GEMM_PLAIN : EPI, true>(tA, tB, tB2, p, grid, st);
+  return launch_g<BN, EPI, false>(tA, tB, tB2, p, grid, st);
 }
 
 template <int EPI>
@@ -1610,7 +1596,7 @@ int moe::router_topk_gemm(const void* x, const void* Wr, int64_t T, int H, int E
   p.b_tx_bytes = E * BK * 2;
   const int64_t tiles = (T + BM - 1) / BM;
   const int grid = (int)(tiles < dev.sm_count ? tiles : dev.sm_count);
-  return launch<1, 128, EPI_ROUTER>(tA, tB, tB, p, grid, st);
+  return launch<128, EPI_ROUTER>(tA, tB, tB, p, grid, st);
 }
 
 int moe::grouped_gemm_scatter_slots(const void* A, const void* B, const int32_t* offsets, const int32_t* dst_rows,
@@ -1665,8 +1651,8 @@ int moe::gemm_splitk_f32(const void* A, const void* B, int64_t T, int K, int N, 
   const int64_t tiles = ((T + BM - 1) / BM) * S;
   const int grid = (int)(tiles < dev.sm_count ? tiles : dev.sm_count);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (N > 128) return launch<1, 256, MOE_GEMM_PLAIN_F32>(tA, tB, tB, p, grid, st);
-  return launch<1, 128, MOE_GEMM_PLAIN_F32>(tA, tB, tB, p, grid, st);
+  if (N > 128) return launch<256, MOE_GEMM_PLAIN_F32>(tA, tB, tB, p, grid, st);
+  return launch<128, MOE_GEMM_PLAIN_F32>(tA, tB, tB, p, grid, st);
 }
 
 extern "C" int moe_grouped_gemm_peer_scatter(const void* A, const void* B, const int32_t* offsets,
@@ -1819,19 +1805,19 @@ static int grouped_gemm_impl(int epilogue, const void* A, const void* B, const v
   int grid = (int)(tiles_bound < dev.sm_count ? tiles_bound : dev.sm_count);
   if (grid < 1) grid = 1;
   if (row_rank) {   // combine exchange fused into the epilogue
-    if (BN == 256) return launch<1, 256, EPI_PEER>(tA, tB, tB2, p, grid, st);
-    return launch<1, 128, EPI_PEER>(tA, tB, tB2, p, grid, st);
+    if (BN == 256) return launch<256, EPI_PEER>(tA, tB, tB2, p, grid, st);
+    return launch<128, EPI_PEER>(tA, tB, tB2, p, grid, st);
   }
 #define MOE_GEMM_CASE(EPI_)                                                                  \
-  if (BN == 256) return launch<1, 256, EPI_>(tA, tB, tB2, p, grid, st);                        \
-  return launch<1, 128, EPI_>(tA, tB, tB2, p, grid, st)
+  if (BN == 256) return launch<256, EPI_>(tA, tB, tB2, p, grid, st);                        \
+  return launch<128, EPI_>(tA, tB, tB2, p, grid, st)
   switch (epilogue) {
     case MOE_GEMM_PLAIN: MOE_GEMM_CASE(MOE_GEMM_PLAIN);
     case MOE_GEMM_SCALE_SCATTER: MOE_GEMM_CASE(MOE_GEMM_SCALE_SCATTER);
     case MOE_GEMM_PLAIN_F32: MOE_GEMM_CASE(MOE_GEMM_PLAIN_F32);
     default:
-      if (few_rows) return launch_g<1, 64, MOE_GEMM_SILU_GATE, true, 32>(tA, tB, tB2, p, grid, st);
-      return launch<1, 256, MOE_GEMM_SILU_GATE>(tA, tB, tB2, p, grid, st);
+      if (few_rows) return launch_g<64, MOE_GEMM_SILU_GATE, true, 32>(tA, tB, tB2, p, grid, st);
+      return launch<256, MOE_GEMM_SILU_GATE>(tA, tB, tB2, p, grid, st);
   }
 #undef MOE_GEMM_CASE
 }
