@@ -95,3 +95,13 @@ def test_shared_group_on_large_batches(cuda, lib, T, E, k, H, I):
     ref = O.fusedmoe(x.cpu(), *[t.cpu() for t in w], k, logits=lg.cpu())
     torch.testing.assert_close(y.float().cpu(), ref, rtol=1e-2, atol=2e-2)
     ops.check_status(cuda)
+
+
+def test_as_many_experts_as_a_gemm_takes(cuda, lib):
+    """1024 routed experts leave no group for the shared one: side-stream form, strided weights through copies as ever."""
+    T, H, I, E = 6, 64, 8, 1024
+    x, w = _inputs(cuda, T, H, I, E, 6)
+    want = _two_streams(x, w, H, I, E, T).clone()
+    turned = [w[0], *(t.mT.contiguous().mT for t in w[1:])]
+    assert torch.equal(_layer(H, I, E, T).forward(x, *turned), want)
+    ops.check_status(cuda)

@@ -135,11 +135,11 @@ class FusedMoETileLang:
     # object holds no copy that a later write to a weight, by whatever means, could leave behind.  Layers whose weights
     # exceed this size keep the side-stream form.
     STACK_LIMIT_BYTES = 2 << 30
-    _stack = None       # (E + 1, I, H) of the experts that the last forward ran as one stack, None for the side-stream form
+    _stack = None       # (E + 1, I, H) of the experts that the last forward took as one stack, None for the side-stream form
 
     def _stack_shape(self, shared_gate, shared_up, shared_down, routed_gate):
         E, I, H = routed_gate.shape
-        if (self.n_shared_experts != 1 or H % 64 or E >= 1024 or shared_gate is None or shared_up is None or shared_down is None
+        if (self.n_shared_experts != 1 or H % 64 or shared_gate is None or shared_up is None or shared_down is None
                 or 3 * (E + 1) * I * H * routed_gate.element_size() > self.STACK_LIMIT_BYTES):
             return None
         return E + 1, I, H
@@ -151,7 +151,7 @@ class FusedMoETileLang:
         if st is not None:
             weights = _stackable((shared_gate, shared_up, shared_down, routed_gate, routed_up, routed_down), st[0] - 1, st[1], st[2])
             return _layer.moe_forward_single_call(x, router_weight, *weights, self.n_experts_per_token, ws=self.ws, logits=logits,
-                                                  shared_group=True)
+                                                  shared_group=st[0] <= 1024)      # groups a grouped GEMM takes
         return _layer.moe_forward_single_call(x, router_weight, shared_gate if self.n_shared_experts else None,
                                               shared_up, shared_down, routed_gate, routed_up, routed_down,
                                               self.n_experts_per_token, ws=self.ws, logits=logits)
