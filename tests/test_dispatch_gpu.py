@@ -95,8 +95,10 @@ def test_few_experts_a_cta_or_a_warp_per_token(cuda, lib, T, H, E, k, dtype):
                                               (32, 320, 264, 16, 8, 0), (33, 2048, 512, 8, 2, 1), (20, 1024, 136, 6, 6, 2)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_up_gemm_of_few_rows(cuda, lib, T, H, I, E, k, shared, dtype):
-    """Up to 32 tokens the layer's up GEMM holds 32 rows of A per stage: the same bits as the wide tiles that the stage-by-stage
-    layer takes (it does not bound the rows of a group), and close to the oracle."""
+    """Up to 32 tokens the layer's up GEMM holds 32 rows of A per stage: close to the oracle, and the same bits as the
+    stage-by-stage layer (whose up GEMM gathers as well but does not know the rows of a group, so it takes the wide tiles
+    where there are more than 32 rows in all) and, for one list of at most 32 rows, as the wide tiles on rows gathered
+    beforehand."""
     from tilelang_moe_b200 import kernels, layer
     x, w = O.make_fusedmoe_inputs(1, T, H, I, E, shared, k, dtype=dtype, seed=T + I)
     names = ["router_weight", "shared_gate", "shared_up", "shared_down", "routed_gate", "routed_up", "routed_down"]
@@ -107,6 +109,9 @@ def test_up_gemm_of_few_rows(cuda, lib, T, H, I, E, k, shared, dtype):
     ref = layer.moe_forward(x.to(cuda), *ws, k, logits=lg.to(cuda))
     ops.check_status(cuda)
     assert torch.equal(y, ref)
+    # the tolerances of the layer tests: 16-bit act, yk and out around fp32 sums
+    exact = O.fusedmoe(x, *[w[n] if shared or not n.startswith("shared") else None for n in names], k, logits=lg)
+    torch.testing.assert_close(y.float().cpu(), exact, rtol=1e-2, atol=2e-2)
     n = min(T, 32)                        # one expert list of at most 32 rows through the generic entry point
     ids = torch.randint(0, E, (n, 1), generator=torch.Generator().manual_seed(T))
     _, offs, perm, _ = O.route_histogram(ids, E)
