@@ -138,8 +138,8 @@ def test_single_call_layer_equals_the_staged_calls(cuda, lib, B, S, H, I, E, NS,
     y0 = layer.moe_forward(xd, *wd, k).clone()
     ops.check_status(cuda)
     assert y1.shape == x.shape and torch.equal(y1, y0)
-    # a single shared expert of the routed width ran as expert E of the routed GEMMs (stacked weights kept by the layer
-    # object); the same layer with the stacking switched off takes the side-stream form: all three agree bit for bit
+    # a single shared expert of the routed width ran as expert E of the routed GEMMs; the same layer with that switched off
+    # takes the side-stream form: all three agree bit for bit
     assert (getattr(m, "_stack", None) is not None) == (NS == 1 and H % 64 == 0)
     if NS == 1:
         m2 = kernels.FusedMoETileLang(H, I, E, NS, k, B, S, dtype=dtype)

@@ -160,7 +160,7 @@ def test_router_gemm_then_topk_like_the_reference_fusion_test(cuda, lib, H, E, K
                                    (2100, 512, 5), (2050, 1024, 8), (2048, 12, 3), (2200, 300, 7), (2304, 128, 1)])
 @pytest.mark.parametrize("mode", ["B", "A", "A_renorm"])
 def test_tile_path_shapes(cuda, lib, M, N, k, mode):
-    """Thread-per-row tile kernel (M >= 2048, k <= 8, aligned rows): 1, 2, 4 or 8 threads per row."""
+    """Lane-group and lane-per-row kernels (M >= 2048, k <= 8, aligned rows): 1 to 32 lanes per row."""
     lg = torch.randn(M, N, generator=torch.Generator().manual_seed(M + N + k))
     _check(lg, k, mode, cuda)
 
