@@ -158,7 +158,7 @@ static int launch_warp(const float* logits, int64_t M, int N, int64_t ld, int k,
 // thread-per-row tiles with a list of K per thread before -> now): 1048576 x 128, k = 6: 169 -> 138 (HBM 93);
 // 131072 x 256, k = 8: 65.7 -> 34.3; 131072 x 1024, k = 8: 291 -> 115 (HBM 84); 16384 x 256: 11.7 -> 6.8; 2048 x 256:
 // 8.8 -> 3.4.  With a few lanes per row 32 warps per SM fit beside each other; the tiles had 12.  Equal logits: 131072 x
-// 128, k = 6 all equal 25.0 -> 21.4, rounded to integers 29.0 -> 24.2; rounded, k = 8: 32768 x 128 13.2 -> 11.2, 131072 x 64
+// 128, k = 6 all equal 25.0 -> 20.8, rounded to integers 29.0 -> 23.6; rounded, k = 8: 32768 x 128 13.2 -> 11.2, 131072 x 64
 // 33.0 -> 20.9.  Slower than the tiles and the warp kernel: rounded to integers, k = 2, 32768 x 36 4.8 -> 6.2, x 100 6.1 -> 6.8 (a
 // dozen entries to rank for two places), and 64 x 300, k = 8 3.9 -> 4.5.
 // ------------------------------------------------------------------------------------
@@ -286,8 +286,7 @@ topk_group_kernel(const float* __restrict__ logits, int64_t M, int N, int64_t ld
     cmax = __reduce_max_sync(FULL, c);
     if (cmax <= CAP) {
       const uint64_t vkey = (uint64_t)float_to_key(V) << 32;
-      const int rounds = __reduce_max_sync(FULL, K - c);
-      for (int r = 0; r < rounds; ++r) {
+      for (int r = 0; r < K; ++r) {                 // a bound known to the compiler: with K - c the kernel was 1 % slower on every row
         const int b = __ffs(eq) - 1;
         const uint32_t col = eq ? (uint32_t)(4 * ((b >> 2) * L + sub) + (b & 3)) : 0xFFFFFFFFu;
         uint32_t first = col;
